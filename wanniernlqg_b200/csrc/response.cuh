@@ -999,18 +999,56 @@ __global__ void __launch_bounds__(WIDE ? 512 : 256, WIDE ? 1 : (sizeof(R) == 8 ?
     }
 }
 
-// out[v] = sum over CTAs g (in order) of partials[g][v], compensated.
-__global__ void reduce_partials_kernel(const double *__restrict__ partials, int64_t nslots, int64_t vc,
-                                       double2 *__restrict__ out) {
-    for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < vc; v += (int64_t)gridDim.x * blockDim.x) {
-        double sr = 0.0, cr = 0.0, si = 0.0, ci = 0.0;
-        for (int64_t g = 0; g < nslots; ++g) {
-            const double *a = partials + (g * vc + v) * 4;
-            neumaier_add(sr, cr, a[0]);
-            neumaier_add(sr, cr, a[2]);
-            neumaier_add(si, ci, a[1]);
-            neumaier_add(si, ci, a[3]);
+// out[v] = sum over slots g of partials[g][v], compensated, in a fixed order.  A block of
+// REDUCE_THREADS takes vx values (at most 8: one slot's 8 values are two whole 128-byte lines) and
+// splits the slots over its REDUCE_THREADS / vx groups: group q sums slots q, q + groups, ... in
+// order, four slots' loads in flight, and a fixed binary tree adds the groups.  Bound by latency:
+// one thread per value over all slots took 653 us for 1184 slots of 256 values (4-orbital mesh) and
+// 167 us for 296 slots of 201 values (cold-cache launch times); this split takes 12.6 and 7.1 us.
+#define REDUCE_THREADS 1024
+WNLQG_HD int reduce_values_per_block(int64_t vc) {
+    int vx = 1;
+    while (vx < 8 && vx < vc) vx <<= 1;
+    return vx;
+}
+
+__global__ void __launch_bounds__(REDUCE_THREADS) reduce_partials_kernel(const double *__restrict__ partials, int64_t nslots,
+                                                                         int64_t vc, double2 *__restrict__ out) {
+    __shared__ double4 part[REDUCE_THREADS];   // (sum re, sum im, comp re, comp im)
+    const int vx = reduce_values_per_block(vc), groups = REDUCE_THREADS / vx;
+    const int q = threadIdx.x / vx;
+    const int64_t v = (int64_t)blockIdx.x * vx + (threadIdx.x & (vx - 1));
+    const double2 *src = reinterpret_cast<const double2 *>(partials);
+    double4 a = make_double4(0.0, 0.0, 0.0, 0.0);
+    auto add = [&](double2 s, double2 c) {
+        neumaier_add(a.x, a.z, s.x);
+        neumaier_add(a.x, a.z, c.x);
+        neumaier_add(a.y, a.w, s.y);
+        neumaier_add(a.y, a.w, c.y);
+    };
+    if (v < vc) {
+        constexpr int B = 4;
+        for (int64_t g0 = q; g0 < nslots; g0 += (int64_t)B * groups) {
+            double2 s[B], c[B];
+#pragma unroll
+            for (int j = 0; j < B; ++j) {
+                const int64_t g = g0 + (int64_t)j * groups;
+                const bool in = g < nslots;
+                s[j] = in ? src[(g * vc + v) * 2] : make_double2(0.0, 0.0);
+                c[j] = in ? src[(g * vc + v) * 2 + 1] : make_double2(0.0, 0.0);
+            }
+#pragma unroll
+            for (int j = 0; j < B; ++j) add(s[j], c[j]);
         }
-        out[v] = make_double2(sr + cr, si + ci);
     }
+    part[threadIdx.x] = a;
+    for (int h = groups >> 1; h > 0; h >>= 1) {   // fixed binary tree over the groups
+        __syncthreads();
+        if (q < h) {
+            const double4 t = part[threadIdx.x + h * vx];
+            add(make_double2(t.x, t.y), make_double2(t.z, t.w));
+            part[threadIdx.x] = a;
+        }
+    }
+    if (q == 0 && v < vc) out[v] = make_double2(a.x + a.z, a.y + a.w);
 }

@@ -2130,6 +2130,16 @@ wnlqg_status order_batch(wnlqg_plan *pl, const double *k, const double *w, int64
     return WNLQG_OK;
 }
 
+// The plan's partial sums, summed over their slots into out (device, value-count complex values).
+wnlqg_status launch_reduce(wnlqg_plan *pl, double2 *out) {
+    const int64_t vx = reduce_values_per_block(pl->vc);
+    reduce_partials_kernel<<<(unsigned)std::max<int64_t>(1, (pl->vc + vx - 1) / vx), REDUCE_THREADS, 0, pl->stream>>>(
+        pl->d_partials, pl->partial_slots, pl->vc, out);
+    pl->launches += 1;
+    WNLQG_CUDA(cudaGetLastError());
+    return WNLQG_OK;
+}
+
 wnlqg_status check_mesh_args(wnlqg_plan *pl, const int64_t mesh[3], int64_t k_begin, int64_t k_end, const double *out) {
     wnlqg_status st = check_plan(pl);
     if (st != WNLQG_OK) return st;
@@ -2172,10 +2182,7 @@ wnlqg_status enqueue_mesh(wnlqg_plan *pl, const int64_t mesh[3], int64_t k_begin
     // next batch start (or the final event) closes the response stage.
     size_t final_ev = 1 + 3 * nbatch;
     if ((st = record_event(pl, final_ev)) != WNLQG_OK) return st;
-    reduce_partials_kernel<<<(unsigned)std::max<int64_t>(1, std::min<int64_t>((pl->vc + 255) / 256, 1024)), 256, 0,
-                             pl->stream>>>(pl->d_partials, pl->partial_slots, pl->vc, reinterpret_cast<double2 *>(out_device));
-    pl->launches += 1;
-    WNLQG_CUDA(cudaGetLastError());
+    if ((st = launch_reduce(pl, reinterpret_cast<double2 *>(out_device))) != WNLQG_OK) return st;
     if ((st = record_event(pl, final_ev + 1)) != WNLQG_OK) return st;
     pl->timing_valid = true;
     pl->timing_batches = nbatch;
@@ -2253,10 +2260,7 @@ wnlqg_status enqueue_points_weighted(wnlqg_plan *pl, const double *kpoints_devic
     }
     const size_t final_ev = 1 + 3 * nbatch;
     if ((st = record_event(pl, final_ev)) != WNLQG_OK) return st;
-    reduce_partials_kernel<<<(unsigned)std::max<int64_t>(1, std::min<int64_t>((pl->vc + 255) / 256, 1024)), 256, 0,
-                             pl->stream>>>(pl->d_partials, pl->partial_slots, pl->vc, reinterpret_cast<double2 *>(out_device));
-    pl->launches += 1;
-    WNLQG_CUDA(cudaGetLastError());
+    if ((st = launch_reduce(pl, reinterpret_cast<double2 *>(out_device))) != WNLQG_OK) return st;
     if ((st = record_event(pl, final_ev + 1)) != WNLQG_OK) return st;
     pl->timing_valid = true;
     pl->timing_batches = nbatch;
@@ -2406,10 +2410,7 @@ wnlqg_status wnlqg_b200_eval_points_weighted(wnlqg_plan *pl, const double *kpoin
         if ((st = run_isolation(pl, nb, s, perm)) != WNLQG_OK) return st;
         if ((st = run_passes(pl, nb, 0, 1.0, 0, ord ? pl->d_ow : pl->d_weights)) != WNLQG_OK) return st;
     }
-    reduce_partials_kernel<<<(unsigned)std::max<int64_t>(1, std::min<int64_t>((pl->vc + 255) / 256, 1024)), 256, 0,
-                             pl->stream>>>(pl->d_partials, pl->partial_slots, pl->vc, pl->d_out);
-    pl->launches += 1;
-    WNLQG_CUDA(cudaGetLastError());
+    if ((st = launch_reduce(pl, pl->d_out)) != WNLQG_OK) return st;
     WNLQG_CUDA(cudaMemcpyAsync(out, pl->d_out, (size_t)pl->vc * sizeof(double2), cudaMemcpyDeviceToHost, pl->stream));
     WNLQG_CUDA(cudaStreamSynchronize(pl->stream));
     pl->timing_valid = false;
@@ -2452,10 +2453,7 @@ wnlqg_status wnlqg_b200_eval_mesh_weighted(wnlqg_plan *pl, const int64_t mesh[3]
         if ((st = run_isolation(pl, nb, s, nullptr)) != WNLQG_OK) return st;
         if ((st = run_passes(pl, nb, 0, 1.0, 0, pl->d_weights)) != WNLQG_OK) return st;
     }
-    reduce_partials_kernel<<<(unsigned)std::max<int64_t>(1, std::min<int64_t>((pl->vc + 255) / 256, 1024)), 256, 0,
-                             pl->stream>>>(pl->d_partials, pl->partial_slots, pl->vc, pl->d_out);
-    pl->launches += 1;
-    WNLQG_CUDA(cudaGetLastError());
+    if ((st = launch_reduce(pl, pl->d_out)) != WNLQG_OK) return st;
     WNLQG_CUDA(cudaMemcpyAsync(out, pl->d_out, (size_t)pl->vc * sizeof(double2), cudaMemcpyDeviceToHost, pl->stream));
     WNLQG_CUDA(cudaStreamSynchronize(pl->stream));
     pl->timing_valid = false;
