@@ -28,7 +28,6 @@ enum { RS_FC_SHIFT = 1, RS_FC_INJECTION = 2, RS_FC_JERK = 3 };
 enum { RS_SC_BERRY = 1, RS_SC_METRIC = 2 };
 enum { RS_MU_AHC = 1, RS_MU_DIPOLE = 2, RS_MU_LT = 3, RS_MU_BANDCURV = 4 };
 #define RS_MAX_HESS 9
-#define RS_MU_CHUNK 8
 
 struct RespParams {
     int nw, ld;
@@ -146,7 +145,7 @@ struct RespSmem {
         s.f = take(nw * sizeof(double));
         s.te = take((size_t)nw * nw * sizeof(double));
         s.fnm = take((size_t)nw * nw * sizeof(double));
-        s.Q = take((size_t)nw * nw * (n_fc > 0 ? n_fc : 1) * csize);
+        s.Q = take((size_t)nw * nw * n_fc * csize);
         s.fd = take((size_t)4 * nw * (n_berry > 0 ? n_berry : 1) * sizeof(double2));
         s.hess = take((size_t)RS_MAX_HESS * nw * sizeof(double));
         s.red = take(64 * sizeof(double) + 64 * sizeof(int));
@@ -371,6 +370,12 @@ WNLQG_D void rotate_diagonal(const double2 *__restrict__ src, C *T1, C *T2, cons
     __syncthreads();
 }
 
+// Sum over a warp by a fixed butterfly, the same value in every lane.
+WNLQG_D double warp_sum(double v) {
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+
 // Deterministic block sum of one double per thread (fixed shuffle tree, warps in order).
 WNLQG_D double block_sum(double v, double *red) {
     for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
@@ -492,8 +497,10 @@ WNLQG_D void contract_dispatch(int pair_mode, int gaussian, const double *ste, c
 // the shared-memory kernel addresses shared memory directly.
 // WIDE: 512 threads per CTA (16 warps to hide the FP64 latencies of the one CTA an SM holds) at
 // 128 registers per thread instead of 256 threads at up to 255; the autotuner picks the width.
-template <typename R, bool NG, bool GW, bool WIDE = false>
-__global__ void __launch_bounds__(WIDE ? 512 : 256, WIDE ? 1 : (sizeof(R) == 8 ? 1 : 2)) response_kernel(RespParams p) {
+// FREQ: passes with frequency components; without them (scalar and Fermi-axis components only) the
+// kernel carries no contraction accumulators and fits two CTAs of 256 threads per SM.
+template <typename R, bool NG, bool GW, bool WIDE = false, bool FREQ = true>
+__global__ void __launch_bounds__(WIDE ? 512 : 256, WIDE ? 1 : (sizeof(R) == 8 && FREQ ? 1 : 2)) response_kernel(RespParams p) {
     typedef typename cplx_of<R>::type C;
     extern __shared__ __align__(16) unsigned char smem_dyn[];
     unsigned char *sm;
@@ -686,23 +693,37 @@ __global__ void __launch_bounds__(WIDE ? 512 : 256, WIDE ? 1 : (sizeof(R) == 8 ?
         }
 
 
-        // Fermi-energy-axis responses.
+        // Fermi-energy-axis responses.  What depends on the pair of bands is formed once per
+        // component in the pair-data region (free until the pairs are built); the Fermi levels then
+        // only combine it: a warp per level (dipole, linear transport) or a thread per level (AHC).
+        // Bound before by barriers and serial sums (a block sum per level, the dipole's levels on one
+        // thread): a 201-level Hall scan of 18 orbitals, 2025 points, took 2.43 ms and takes 0.70;
+        // transport and dipole at 3 levels, 24 orbitals, 32768 points, 21.2 ms and 11.6.
+        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+        auto mu_emit = [&](int64_t idx, double value) {
+            if (p.mode == 0) {
+                double *a4 = p.partials + ((int64_t)blockIdx.x * p.vc + idx) * 4;
+                neumaier_add(a4[0], a4[2], value * wk);
+            } else {
+                p.out_points[(p.point_offset + (p.out_perm ? (int64_t)p.out_perm[b] : (int64_t)b)) * p.vc + idx] = make_double2(value * p.scale, 0.0);
+            }
+        };
         for (int s = 0; s < p.n_mu; ++s) {
             const int a = p.mu_a[s], bb = p.mu_b[s], cc = p.mu_c[s];
-            // F_nn^{ab} (Hamiltonian-gauge Wannier curvature diagonal) into sFd[2nw .. 3nw).
-            rotate_diagonal(xw + (int64_t)p.ch_dA[bb * 3 + a] * nn, T1, T2, sU, sFd, nw, ld,
-                            xw + (int64_t)p.ch_dA[a * 3 + bb] * nn);
-            for (int n = threadIdx.x; n < nw; n += blockDim.x) sFd[nw + n] = make_double2(0.0, 0.0);
-            __syncthreads();
-            const C *Aa = slot(p.slot_A[a]), *Ab = slot(p.slot_A[bb]);
-            const C *Ha = slot(p.slot_dH[a]), *Hb = slot(p.slot_dH[bb]);
-            band_sums(
-                nw,
-                [&](int n, int l) {
-                    return to_c64(csub(cmul(Aa[n + ld * l], Ab[l + ld * n]), cmul(Ab[n + ld * l], Aa[l + ld * n])));
-                },
-                [&](int n, double2 comm) { sFd[2 * nw + n] = csub(csub(sFd[n], sFd[nw + n]), cmuli(comm)); });
-            __syncthreads();
+            if (s == 0 || p.mu_a[s - 1] != a || p.mu_b[s - 1] != bb) {
+                // F_nn^{ab} (Hamiltonian-gauge Wannier curvature diagonal) into sFd[2nw .. 3nw); the
+                // next component of the same (a, b) finds it there.
+                rotate_diagonal(xw + (int64_t)p.ch_dA[bb * 3 + a] * nn, T1, T2, sU, sFd, nw, ld,
+                                xw + (int64_t)p.ch_dA[a * 3 + bb] * nn);
+                const C *Aa = slot(p.slot_A[a]), *Ab = slot(p.slot_A[bb]);
+                band_sums(
+                    nw,
+                    [&](int n, int l) {
+                        return to_c64(csub(cmul(Aa[n + ld * l], Ab[l + ld * n]), cmul(Ab[n + ld * l], Aa[l + ld * n])));
+                    },
+                    [&](int n, double2 comm) { sFd[2 * nw + n] = csub(sFd[n], cmuli(comm)); });
+                __syncthreads();
+            }
             if (p.mu_kind[s] == RS_MU_BANDCURV) {
                 // berry_curvature_group_sum_component with the group {n} (ConventionalQuantumGeometry.jl:
                 // 530-557): Re F_nn + sum_{m != n} -Im(r^a_nm r^b_mn - r^b_nm r^a_mn).
@@ -718,124 +739,122 @@ __global__ void __launch_bounds__(WIDE ? 512 : 256, WIDE ? 1 : (sizeof(R) == 8 ?
                 __syncthreads();
             } else if (p.mu_kind[s] == RS_MU_DIPOLE) {
                 // Band Berry curvature Omega_n = -2 sum_m Im(r^a_nm r^b_mn) + Re F_nn
-                // (berry_curvature_component, ConventionalQuantumGeometry.jl:166-180) into sFd[3nw..).
+                // (berry_curvature_component, ConventionalQuantumGeometry.jl:166-180) and the band
+                // velocity into sFd[3nw..).
+                const C *Hc = slot(p.slot_dH[cc]);
                 band_sums(
                     nw,
                     [&](int n, int m) {
                         if (m == n) return make_double2(0.0, 0.0);
                         return make_double2(-to_c64(cmul(r_elem(a, n, m), r_elem(bb, m, n))).y, 0.0);
                     },
-                    [&](int n, double2 om) { sFd[3 * nw + n] = make_double2(2.0 * om.x + sFd[2 * nw + n].x, 0.0); });
+                    [&](int n, double2 om) {
+                        sFd[3 * nw + n] = make_double2(2.0 * om.x + sFd[2 * nw + n].x, (double)Hc[n + ld * n].x);
+                    });
                 __syncthreads();
-                if (threadIdx.x == 0) {
-                    const C *Hc = slot(p.slot_dH[cc]);
-                    for (int im = 0; im < p.nmu; ++im) {
-                        const double mu = p.mus[im];
-                        double value = 0.0;
-                        for (int n = 0; n < nw; ++n) {
-                            double w;
-                            if (p.temperature > 0.0) {
-                                const double scale = 8.617333262145e-5 * p.temperature;
-                                const double z = exp(-fabs((sE[n] - mu) / scale));
-                                w = z / (scale * (1.0 + z) * (1.0 + z));
-                            } else {
-                                const double x = (sE[n] - mu) / p.fs_width;
-                                w = exp(-x * x) / (sqrt(WNLQG_PI) * p.fs_width);
-                            }
-                            value += w * sFd[3 * nw + n].x * (double)Hc[n + ld * n].x;
-                        }
-                        const int64_t idx = p.mu_out[s] + im;
-                        if (p.mode == 0) {
-                            double *a4 = p.partials + ((int64_t)blockIdx.x * p.vc + idx) * 4;
-                            neumaier_add(a4[0], a4[2], value * wk);
+                for (int im = warp; im < p.nmu; im += nwarps) {
+                    const double mu = p.mus[im];
+                    double value = 0.0;
+                    for (int n = lane; n < nw; n += 32) {
+                        double w;
+                        if (p.temperature > 0.0) {
+                            const double scale = 8.617333262145e-5 * p.temperature;
+                            const double z = exp(-fabs((sE[n] - mu) / scale));
+                            w = z / (scale * (1.0 + z) * (1.0 + z));
                         } else {
-                            p.out_points[(p.point_offset + (p.out_perm ? (int64_t)p.out_perm[b] : (int64_t)b)) * p.vc + idx] = make_double2(value * p.scale, 0.0);
+                            const double x = (sE[n] - mu) / p.fs_width;
+                            w = exp(-x * x) / (sqrt(WNLQG_PI) * p.fs_width);
                         }
+                        value += w * sFd[3 * nw + n].x * sFd[3 * nw + n].y;
                     }
+                    value = warp_sum(value);
+                    if (lane == 0) mu_emit(p.mu_out[s] + im, value);
+                }
+                __syncthreads();
+            } else if (p.mu_kind[s] == RS_MU_LT) {
+                // Berry channel of _linear_transport_response (LinearTransportKernels.jl:100-163):
+                // contact -f(E_l) Re F_ll and, over ordered pairs of distinct spectral blocks,
+                // (f_l - f_m) gap^2/(gap^2 + gamma^2) Im(r^a_lm r^b_ml) (both orders give the
+                // reference's 2 Im q of each unordered pair); the common factor -e^2/hbar 1e-20 is
+                // applied to the sum.  Spectral blocks: levels within 32 eps max(1, max|E|).
+                double exact = 0.0;
+                for (int n = 0; n < nw; ++n) exact = fmax(exact, fabs(sE[n]));
+                exact = 32.0 * 2.220446049250313e-16 * fmax(1.0, exact);
+                for (int e = threadIdx.x; e < nn; e += blockDim.x) {
+                    const int l = e % nw, m = e / nw;
+                    const double gap = sE[m] - sE[l];
+                    const bool joined = l == m || fabs(gap) <= exact;
+                    const double rate = gap * gap / (gap * gap + p.lt_gamma * p.lt_gamma);
+                    ste[e] = joined ? 0.0 : rate * cmuli(to_c64(cmul(r_elem(a, l, m), r_elem(bb, m, l)))).x;
+                }
+                __syncthreads();
+                double *focc = sfnm + warp * nw;   // nwarps nw <= nn: see response_threads
+                for (int im = warp; im < p.nmu; im += nwarps) {
+                    const double mu = p.mus[im];
+                    for (int n = lane; n < nw; n += 32) focc[n] = response_occ(sE[n], mu, p.temperature);
+                    __syncwarp();
+                    double value = 0.0;
+                    for (int l = lane; l < nw; l += 32) {
+                        const double fl = focc[l];
+                        double v = fl * sFd[2 * nw + l].x;
+                        for (int m = 0; m < nw; ++m) v += (fl - focc[m]) * ste[l + nw * m];
+                        value += v;
+                    }
+                    value = warp_sum(value);
+                    if (lane == 0) mu_emit(p.mu_out[s] + im, -p.lt_factor * value);
+                    __syncwarp();
                 }
                 __syncthreads();
             } else {
-                for (int m0 = 0; m0 < p.nmu; m0 += RS_MU_CHUNK) {
-                    double loc[RS_MU_CHUNK];
-                    int nocc[RS_MU_CHUNK];
-#pragma unroll
-                    for (int j = 0; j < RS_MU_CHUNK; ++j) {
-                        loc[j] = 0.0;
-                        nocc[j] = 0;
-                        if (m0 + j < p.nmu) {
-                            const double mu = p.mus[m0 + j];
-                            for (int n = 0; n < nw; ++n) nocc[j] += sE[n] <= mu ? 1 : 0;
-                        }
+                // Zero temperature (the only AHC temperature, checked at plan creation): matrix
+                // curvature with bare occupied/empty links (IntrinsicHallCurvature.jl:2-29,
+                // IntrinsicHallGeometry.jl:117-136).  The value depends on a Fermi level only through
+                // the number c of levels at or below it, so the sums of every c = 0 .. nw (a warp
+                // each) replace one sum per Fermi level.
+                for (int e = threadIdx.x; e < nn; e += blockDim.x) {
+                    const int l = e % nw, m = e / nw;
+                    double pair = 0.0;
+                    if (l != m) {
+                        const double g = sE[l] - sE[m];
+                        auto link = [&](int ax, int x, int y, double inv) {
+                            const double2 A = to_c64(slot(p.slot_A[ax])[x + ld * y]);
+                            const double2 H = to_c64(slot(p.slot_dH[ax])[x + ld * y]);
+                            return cadd(A, cmuli(cscale(H, -inv)));
+                        };
+                        const double ilm = 1.0 / g, iml = -1.0 / g;
+                        const double2 left = cmul(link(a, l, m, ilm), link(bb, m, l, iml));
+                        const double2 right = cmul(link(bb, l, m, ilm), link(a, m, l, iml));
+                        pair = -(left.y - right.y);
                     }
-                    double exact = 0.0;   // spectral blocks: levels within 32 eps max(1, max|E|)
-                    if (p.mu_kind[s] == RS_MU_LT) {
-                        for (int n = 0; n < nw; ++n) exact = fmax(exact, fabs(sE[n]));
-                        exact = 32.0 * 2.220446049250313e-16 * fmax(1.0, exact);
-                    }
-                    for (int e = threadIdx.x; e < nn; e += blockDim.x) {
-                        const int l = e % nw, m = e / nw;
-                        if (p.mu_kind[s] == RS_MU_LT) {
-                            // Berry channel of _linear_transport_response (LinearTransportKernels.jl:
-                            // 100-163): contact -f(E_l) Re F_ll and, over ordered pairs of distinct
-                            // spectral blocks, (f_l - f_m) gap^2/(gap^2 + gamma^2) Im(r^a_lm r^b_ml)
-                            // (both orders give the reference's 2 Im q of each unordered pair); the
-                            // common factor -e^2/hbar 1e-20 is applied to the sum.
-                            const double gap = sE[m] - sE[l];
-                            const bool joined = l != m && fabs(gap) <= exact;
-                            const double rate = gap * gap / (gap * gap + p.lt_gamma * p.lt_gamma);
-                            const double2 t = (l == m || joined)
-                                                  ? make_double2(0.0, 0.0)
-                                                  : cmuli(to_c64(cmul(r_elem(a, l, m), r_elem(bb, m, l))));
-#pragma unroll
-                            for (int j = 0; j < RS_MU_CHUNK; ++j) {
-                                if (m0 + j >= p.nmu) continue;
-                                const double mu = p.mus[m0 + j];
-                                const double fl = response_occ(sE[l], mu, p.temperature);
-                                if (l == m) loc[j] += fl * sFd[2 * nw + l].x;
-                                else if (!joined) loc[j] += (fl - response_occ(sE[m], mu, p.temperature)) * rate * t.x;
-                            }
-                        } else {
-                            // Zero temperature (the only AHC temperature, checked at plan creation):
-                            // matrix curvature with bare occupied/empty links
-                            // (IntrinsicHallCurvature.jl:2-29, IntrinsicHallGeometry.jl:117-136).
-                            double pair = 0.0;
-                            if (l != m) {
-                                const double g = sE[l] - sE[m];
-                                auto link = [&](int ax, int x, int y, double inv) {
-                                    const double2 A = to_c64(slot(p.slot_A[ax])[x + ld * y]);
-                                    const double2 H = to_c64(slot(p.slot_dH[ax])[x + ld * y]);
-                                    return cadd(A, cmuli(cscale(H, -inv)));
-                                };
-                                const double ilm = 1.0 / g, iml = -1.0 / g;
-                                const double2 left = cmul(link(a, l, m, ilm), link(bb, m, l, iml));
-                                const double2 right = cmul(link(bb, l, m, ilm), link(a, m, l, iml));
-                                pair = -(left.y - right.y);
-                            }
-#pragma unroll
-                            for (int j = 0; j < RS_MU_CHUNK; ++j) {
-                                if (m0 + j >= p.nmu) continue;
-                                if (l == m) { if (l < nocc[j]) loc[j] += sFd[2 * nw + l].x; }
-                                else if (l < nocc[j] && m >= nocc[j]) loc[j] += pair;
-                            }
-                        }
-                    }
-                    const double mu_scale = p.mu_kind[s] == RS_MU_LT ? -p.lt_factor : 1.0;
-                    for (int j = 0; j < RS_MU_CHUNK && m0 + j < p.nmu; ++j) {
-                        const double total = mu_scale * block_sum(loc[j], red);
-                        if (threadIdx.x == 0) {
-                            const int64_t idx = p.mu_out[s] + m0 + j;
-                            if (p.mode == 0) {
-                                double *a4 = p.partials + ((int64_t)blockIdx.x * p.vc + idx) * 4;
-                                neumaier_add(a4[0], a4[2], total * wk);
-                            } else {
-                                p.out_points[(p.point_offset + (p.out_perm ? (int64_t)p.out_perm[b] : (int64_t)b)) * p.vc + idx] = make_double2(total * p.scale, 0.0);
-                            }
-                        }
-                    }
+                    ste[e] = pair;
                 }
+                __syncthreads();
+                for (int c = warp; c <= nw; c += nwarps) {
+                    double value = 0.0;
+                    for (int l = lane; l < c; l += 32) {
+                        double v = sFd[2 * nw + l].x;
+                        for (int m = c; m < nw; ++m) v += ste[l + nw * m];
+                        value += v;
+                    }
+                    value = warp_sum(value);
+                    if (lane == 0) sfnm[c] = value;
+                }
+                __syncthreads();
+                for (int im = threadIdx.x; im < p.nmu; im += blockDim.x) {
+                    const double mu = p.mus[im];
+                    int lo = 0, hi = nw;   // energies ascend
+                    while (lo < hi) {
+                        const int mid = (lo + hi) >> 1;
+                        if (sE[mid] <= mu) lo = mid + 1;
+                        else hi = mid;
+                    }
+                    mu_emit(p.mu_out[s] + im, sfnm[lo]);
+                }
+                __syncthreads();
             }
         }
 
+        if constexpr (FREQ) {
         // Band Hessians for jerk: H_n^{ad} = Re ddH_ad[n,n] + 2 sum_{l!=n} Re(dH_a[n,l] dH_d[l,n]) reg(E_n-E_l)
         // (prepare_third_order_band_geometry!, ThirdOrderGeometry.jl:131-160).
         for (int h = 0; h < p.n_hess; ++h) {
@@ -994,6 +1013,7 @@ __global__ void __launch_bounds__(WIDE ? 512 : 256, WIDE ? 1 : (sizeof(R) == 8 ?
                     }
                 }
             }
+        }
         }
         __syncthreads();
     }

@@ -283,7 +283,11 @@ cudaError_t allow_dynamic_smem(const void *fn, int smem_optin) {
 const void *response_wide_fn() { return (const void *)response_kernel<double, false, false, true>; }
 
 // The response kernel instantiation for a precision, a geometry source and a working-set location.
-const void *response_fn(bool mixed, bool nonorth, bool global) {
+const void *response_fn(bool mixed, bool nonorth, bool global, bool freq) {
+    if (!freq && !nonorth) {
+        if (mixed) return global ? (const void *)response_kernel<float, false, true, false, false> : (const void *)response_kernel<float, false, false, false, false>;
+        return global ? (const void *)response_kernel<double, false, true, false, false> : (const void *)response_kernel<double, false, false, false, false>;
+    }
     if (mixed) {
         if (nonorth) return global ? (const void *)response_kernel<float, true, true> : (const void *)response_kernel<float, true, false>;
         return global ? (const void *)response_kernel<float, false, true> : (const void *)response_kernel<float, false, false>;
@@ -354,8 +358,8 @@ wnlqg_status build_passes(wnlqg_plan *pl, int sm_count, size_t smem_limit) {
     const int csize = mixed ? (int)sizeof(float2) : (int)sizeof(double2);
     {
         cudaError_t e = cudaSuccess;
-        for (int v = 0; v < 4 && e == cudaSuccess; ++v)
-            e = allow_dynamic_smem(response_fn(v & 1, v & 2, false), (int)smem_limit);
+        for (int v = 0; v < 8 && e == cudaSuccess; ++v)
+            e = allow_dynamic_smem(response_fn(v & 1, v & 2, false, v & 4), (int)smem_limit);
         if (e == cudaSuccess) e = allow_dynamic_smem(response_wide_fn(), (int)smem_limit);
         if (e != cudaSuccess) return fail(WNLQG_ERR_CUDA, std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(e));
     }
@@ -518,13 +522,13 @@ wnlqg_status build_passes(wnlqg_plan *pl, int sm_count, size_t smem_limit) {
         ps.threads = response_threads(pl->nw);
         int per_sm = 0;
         const size_t launch_smem = pass_global ? 0 : ps.smem;
-        cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, response_fn(mixed, pl->nonorth, pass_global),
+        cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, response_fn(mixed, pl->nonorth, pass_global, p.n_fc > 0),
                                                                       ps.threads, launch_smem);
         if (e != cudaSuccess) return fail(WNLQG_ERR_CUDA, std::string("occupancy query: ") + cudaGetErrorString(e));
         if (per_sm < 1) return fail(WNLQG_ERR_UNSUPPORTED, "response kernel cannot be resident with its shared memory");
         ps.grid = sm_count * per_sm;
         if (pass_global) ps.grid = l2_resident_grid(ps.grid, (int64_t)ps.smem, sm_count);
-        if (!mixed && !pl->nonorth && !pass_global && ps.threads == 256) {
+        if (!mixed && !pl->nonorth && !pass_global && p.n_fc > 0 && ps.threads == 256) {
             int per_sm_w = 0;
             e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_w, response_wide_fn(), 512, ps.smem);
             if (e != cudaSuccess) return fail(WNLQG_ERR_CUDA, std::string("occupancy query: ") + cudaGetErrorString(e));
@@ -1038,7 +1042,7 @@ wnlqg_status launch_pass(wnlqg_plan *pl, const Pass &ps, int64_t nb, int mode, d
     if (pl->resp_wide && ps.grid_wide > 0)
         WNLQG_CUDA(cudaLaunchKernel(response_wide_fn(), dim3(ps.grid_wide), dim3(512), args, launch_smem, pl->stream));
     else
-        WNLQG_CUDA(cudaLaunchKernel(response_fn(pl->task.precision == WNLQG_PRECISION_MIXED, pl->nonorth, ps.global),
+        WNLQG_CUDA(cudaLaunchKernel(response_fn(pl->task.precision == WNLQG_PRECISION_MIXED, pl->nonorth, ps.global, p.n_fc > 0),
                                     dim3(ps.global && pl->resp_gw_grid > 0 ? pl->resp_gw_grid : ps.grid),
                                     dim3(ps.threads), args, launch_smem, pl->stream));
     pl->launches += 1;
