@@ -1,0 +1,59 @@
+"""The register eigensolvers at their edges: every padded order up to 32 (odd counts, one orbital, the
+largest order of each group width, the FP64 kernel up to 16 and the FP32 stage from 17), fewer and
+more points than the groups of a warp and of the grid, and exactly degenerate levels, against the
+oracle's energies and the eigenvector residual."""
+import numpy as np
+import pytest
+
+from wanniernlqg_b200 import _abi
+from wanniernlqg_b200.model import TightBindingModel, kramers_doubled_model, synthetic_orthogonal_model
+
+pytestmark = pytest.mark.gpu
+
+
+def bloch(model, k):
+    ph = np.exp(2j * np.pi * (model.r_vectors.T @ k)) / model.r_degeneracies
+    return np.einsum("ijr,r->ij", model.hamiltonian_r, ph)
+
+
+def check(model, k, vectors_for):
+    from wanniernlqg_b200.engine import ResponseEngine
+    task = _abi.TaskArrays([(_abi.QUANTUM_METRIC, ["xx"])])
+    with ResponseEngine(model, task, max_batch=max(64, len(k))) as eng:
+        e, u = eng.spectrum(k)
+    for i in vectors_for:
+        h = bloch(model, k[i])
+        scale = np.linalg.norm(h)
+        assert np.max(np.abs(e[i] - np.linalg.eigvalsh(h))) <= 1e-13 * scale
+        assert np.max(np.abs(h @ u[i] - u[i] * e[i])) <= 1e-12 * scale
+        assert np.max(np.abs(u[i].conj().T @ u[i] - np.eye(model.num_orbitals))) < 1e-12
+        pivot = np.argmax(np.abs(u[i]), axis=0)
+        top = u[i][pivot, np.arange(model.num_orbitals)]
+        assert np.max(np.abs(top.imag)) < 1e-12 and np.min(top.real) > 0
+
+
+@pytest.mark.parametrize("nw", [1, 2, 3, 4, 5, 7, 8, 9, 11, 13, 16, 17, 19, 22, 23, 26, 28, 29, 31, 32])
+def test_every_order(nw):
+    model = synthetic_orthogonal_model(nw, 1, seed=100 + nw, full_position=True)
+    check(model, np.random.default_rng(nw).random((7, 3)), range(7))
+
+
+@pytest.mark.parametrize("nw", [4, 6, 16, 20])
+@pytest.mark.parametrize("points", [1, 3, 33, 5003])
+def test_point_counts(nw, points):
+    model = synthetic_orthogonal_model(nw, 1, seed=7 + nw)
+    check(model, np.random.default_rng(points).random((points, 3)), {0, points // 2, points - 1})
+
+
+@pytest.mark.parametrize("nw", [6, 14, 24])
+def test_degenerate_levels(nw):
+    base = synthetic_orthogonal_model(nw // 2, 1, seed=3, full_position=True)
+    check(kramers_doubled_model(base, 0.0), np.random.default_rng(5).random((6, 3)), range(6))
+
+
+def test_diagonal_and_zero_matrices():
+    ham = np.zeros((5, 5, 1), dtype=complex, order="F")
+    one = TightBindingModel(np.eye(3), np.zeros((3, 1), int), np.ones(1, int), ham, np.zeros((5, 5, 3, 1), complex))
+    check(one, np.zeros((2, 3)), range(2))
+    one.hamiltonian_r[:, :, 0] = np.diag([3.0, -1.0, 2.0, 2.0, 0.5])
+    check(one, np.zeros((2, 3)), range(2))

@@ -237,13 +237,15 @@ __global__ void __launch_bounds__(256, 4) jacobi_eigh_kernel(const double2 *__re
 }
 
 // ---------------------------------------------------------------------------------------------
-// Mixed-precision eigensolver, one team of TEAM threads per matrix, in two kernels:
-//   stage 1 (jacobi_f32_team_kernel): FP32 parallel Jacobi until the off-diagonal norm is below
-//     2^-17 ||H||, warm-started along runs of consecutive mesh points from the previous point's
-//     eigenvectors (V <- V (3I - V^H V)/2, A <- V^H H V);
-//   stage 2 (eigh_refine_f64_team_kernel): FP64 Rayleigh-Ritz refinement, W = second-order
-//     Loewdin orthonormalisation of V, H' = W^H H W, FP64 Jacobi sweeps (quadratic
-//     convergence), U = W J, ascending order and canonical phases.
+// Mixed-precision eigensolver up to 32 orbitals, in two kernels:
+//   stage 1: FP32 parallel Jacobi until the off-diagonal norm is below 2^-17 ||H||, warm-started
+//     along runs of consecutive mesh points from the previous point's eigenvectors (V <- V (3I -
+//     V^H V)/2, A <- V^H H V): on the FP64 path jacobi_f32_reg_kernel (regjacobi.cuh, the matrix in
+//     registers; up to 16 orbitals that path takes one FP64 kernel instead of the two stages), on the
+//     mixed path jacobi_f32_team_kernel (run_orth_eigen says why);
+//   stage 2 (eigh_refine_f64_team_kernel): FP64 Rayleigh-Ritz refinement by one team of TEAM threads
+//     per matrix, W = second-order Loewdin orthonormalisation of V, H' = W^H H W, FP64 Jacobi sweeps
+//     (quadratic convergence), U = W J, ascending order and canonical phases.
 // A team is one warp (TEAM = 32: several teams per CTA, synchronised with __syncwarp) or one
 // CTA of 64 or 128 threads (two or four warps share a matrix, synchronised with __syncthreads;
 // each thread then holds a half or a quarter of a column in the products and does that share of
@@ -297,9 +299,6 @@ struct WarpJacobiSmem {
 
 // One team-synchronous parallel-Jacobi sweep (np - 1 rounds); returns true (in every thread)
 // when a rotation was applied.
-WNLQG_D float recip_sqrt(float x) { return rsqrtf(x); }
-WNLQG_D double recip_sqrt(double x) { return 1.0 / sqrt(x); }
-
 template <typename T, int TEAM>
 WNLQG_D bool team_jacobi_sweep(typename cplx_of<T>::type *A, typename cplx_of<T>::type *V, int np, int ld, T tol,
                                typename cplx_of<T>::type *rot_s, T *rot_c) {
@@ -355,7 +354,7 @@ WNLQG_D bool team_jacobi_sweep(typename cplx_of<T>::type *A, typename cplx_of<T>
                     const T app = A[p + ld * p].x, aqq = A[q + ld * q].x;
                     const T theta = (aqq - app) / ((T)2 * g);
                     const T tt = (theta >= (T)0 ? (T)1 : (T)-1) / (fabs(theta) + sqrt(theta * theta + (T)1));
-                    c = recip_sqrt(tt * tt + (T)1);
+                    c = (T)1 / sqrt(tt * tt + (T)1);
                     const T sn = tt * c;
                     sp.x = sn * (apq.x / g);
                     sp.y = sn * (apq.y / g);

@@ -1,0 +1,400 @@
+// regjacobi.cuh - Hermitian Jacobi with the matrix in registers: one group of lanes per matrix, lane i
+// holding row i of A and of the eigenvectors V, for orders up to 16 (FP64) and 18 to 32 (FP32).
+//
+// The rounds are those of the shared-memory sweeps (eigh.cuh): the circle method pairs the np indices
+// (np even), and A <- J^H A J, V <- V J per round.  Columns are kept in slots: slot 0 holds index 0,
+// slot s >= 1 index ((s - 1 + round) mod (np - 1)) + 1, and the pair k of a round is slots k and
+// np - 1 - k, so that every register index is static; after each round the contents of slots
+// 1 .. np - 1 move down by one.  A round is
+//   - the rotation of each pair, computed by the two lanes that own its rows (the diagonal is kept in
+//     one register per lane, the pair's element is selected from the row by its slot) and passed to the
+//     other lanes through shared memory (np / 2 broadcast reads);
+//   - the column rotations of A and V, lane-local;
+//   - the row rotations of A: each lane exchanges its row with its partner's by shuffles.
+// There is no barrier beyond __syncwarp, and shared memory carries the np / 2 rotations only; the
+// shared-memory form moved both matrices through it twice per round, with two block barriers.
+// Order np <= 16 puts two groups of 16 lanes (np <= 8: four of 8, np <= 4: eight of 4) in a warp.
+#pragma once
+#include "common.cuh"
+
+template <int NP> struct RegGroup {
+    static_assert(NP >= 2 && NP <= 32 && NP % 2 == 0, "even orders up to 32");
+    static constexpr int LANES = NP <= 4 ? 4 : (NP <= 8 ? 8 : (NP <= 16 ? 16 : 32));
+    static constexpr int PER_WARP = 32 / LANES;
+    static WNLQG_D int lane() { return threadIdx.x & (LANES - 1); }
+    static WNLQG_D int group() { return (threadIdx.x & 31) / LANES; }
+    template <typename T> static WNLQG_D T from(T v, int src) { return __shfl_sync(0xffffffffu, v, src, LANES); }
+    template <typename T> static WNLQG_D T sum(T v) {
+#pragma unroll
+        for (int o = LANES / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o, LANES);
+        return v;
+    }
+    // Whether v holds in any lane of this lane's group.
+    static WNLQG_D bool any(bool v) {
+        const unsigned m = __ballot_sync(0xffffffffu, v);
+        return ((m >> (group() * LANES)) & (LANES == 32 ? 0xffffffffu : (1u << (LANES & 31)) - 1u)) != 0;
+    }
+};
+
+template <typename T> struct alignas(16) RegRot { T c, sx, sy, pad; };
+
+WNLQG_D float reg_rsqrt(float x) { return rsqrtf(x); }
+WNLQG_D double reg_rsqrt(double x) { return rsqrt(x); }
+WNLQG_D float reg_rcp(float x) { return __frcp_rn(x); }
+WNLQG_D double reg_rcp(double x) { return 1.0 / x; }
+
+// out = a[sel], 0 <= sel < N, by a tree of selects (static register indices).
+template <int N, typename C> WNLQG_D C reg_select(const C *a, int sel) {
+    C t[N];
+#pragma unroll
+    for (int j = 0; j < N; ++j) t[j] = a[j];
+    int n = N;
+#pragma unroll
+    for (int bit = 1; bit < N; bit <<= 1) {
+        const bool odd = sel & bit;
+        const int m = (n + 1) / 2;
+#pragma unroll
+        for (int j = 0; j < m; ++j) {
+            if (2 * j + 1 < n) {
+                t[j].x = odd ? t[2 * j + 1].x : t[2 * j].x;
+                t[j].y = odd ? t[2 * j + 1].y : t[2 * j].y;
+            } else {
+                t[j] = t[2 * j];
+            }
+        }
+        n = m;
+    }
+    return t[0];
+}
+
+// One sweep (NP - 1 rounds) of the group's matrix: a, v rows of A and V, d the diagonal element of
+// this lane's index.  Elements with |a_pq| <= tol are left.  rot: 2 x NP / 2 rotations of the group's
+// shared memory.  Slot s holds index s at entry and exit.  Returns whether the group rotated.
+template <typename T, int NP>
+WNLQG_D bool reg_jacobi_sweep(typename cplx_of<T>::type (&a)[NP], typename cplx_of<T>::type (&v)[NP], T &d, T tol,
+                              RegRot<T> *rot) {
+    typedef typename cplx_of<T>::type C;
+    typedef RegGroup<NP> G;
+    constexpr int H = NP / 2;
+    const int i = G::lane();
+    const bool active = i < NP;
+    int pos = active ? i : 0;   // slot of this lane's index
+    bool rotated = false;
+#pragma unroll 1
+    for (int round = 0; round < NP - 1; ++round) {
+        const int ps = NP - 1 - pos;   // the partner's slot and index
+        int partner = ps - 1 + round;
+        if (partner >= NP - 1) partner -= NP - 1;
+        partner = ps == 0 ? 0 : partner + 1;
+        if (!active) partner = i;
+        const bool upper = pos >= H;
+        // beta = A[upper index, lower index] from the upper lane's row.
+        const C own = reg_select<H>(a, upper ? ps : 0);
+        C beta;
+        beta.x = G::from(own.x, partner);
+        beta.y = G::from(own.y, partner);
+        if (upper) beta = own;
+        const T dp = G::from(d, partner);
+        const T g2 = beta.x * beta.x + beta.y * beta.y;
+        T c = (T)1;
+        C s = czero<C>();   // x' = c x - conj(s) y, y' = s x + c y for the lower slot x and the upper y
+        if (active && g2 > tol * tol) {
+            const T ginv = reg_rsqrt(g2);
+            const T theta = (upper ? d - dp : dp - d) * ((T)0.5 * ginv);
+            const T tt = copysign(reg_rcp(fabs(theta) + sqrt(theta * theta + (T)1)), theta);
+            c = reg_rsqrt(tt * tt + (T)1);
+            const T sg = tt * c * ginv;
+            s.x = sg * beta.x;
+            s.y = -sg * beta.y;
+            const T shift = tt * (g2 * ginv);
+            d += upper ? shift : -shift;
+            rotated = true;
+        }
+        RegRot<T> *r = rot + (round & 1) * H;
+        if (active && !upper) {
+            RegRot<T> q;
+            q.c = c; q.sx = s.x; q.sy = s.y; q.pad = (T)0;
+            r[pos] = q;
+        }
+        __syncwarp();
+        auto columns = [&](C &x, C &y, const RegRot<T> &q) {
+            const C x0 = x, y0 = y;
+            x.x = fma(-q.sy, y0.y, fma(-q.sx, y0.x, q.c * x0.x));
+            x.y = fma(q.sy, y0.x, fma(-q.sx, y0.y, q.c * x0.y));
+            y.x = fma(-q.sy, x0.y, fma(q.sx, x0.x, q.c * y0.x));
+            y.y = fma(q.sy, x0.x, fma(q.sx, x0.y, q.c * y0.y));
+        };
+#pragma unroll
+        for (int k = 0; k < H; ++k) {
+            const RegRot<T> q = r[k];
+            columns(a[k], a[NP - 1 - k], q);
+            columns(v[k], v[NP - 1 - k], q);
+        }
+        // Row rotation: lower row <- c own - s partner, upper row <- c own + conj(s) partner.
+        const T wx = upper ? s.x : -s.x, wy = -s.y;
+#pragma unroll
+        for (int j = 0; j < NP; ++j) {
+            const T px = G::from(a[j].x, partner), py = G::from(a[j].y, partner);
+            a[j].x = fma(-wy, py, fma(wx, px, c * a[j].x));
+            a[j].y = fma(wy, px, fma(wx, py, c * a[j].y));
+        }
+        if constexpr (NP > 2) {
+            const C a1 = a[1], v1 = v[1];
+#pragma unroll
+            for (int j = 1; j < NP - 1; ++j) { a[j] = a[j + 1]; v[j] = v[j + 1]; }
+            a[NP - 1] = a1;
+            v[NP - 1] = v1;
+            if (active && i > 0) pos = pos == 1 ? NP - 1 : pos - 1;
+        }
+    }
+    return G::any(rotated);
+}
+
+// Squared off-diagonal norm of the group's matrix (slot s holding index s).
+template <typename T, int NP> WNLQG_D T reg_offdiag2(const typename cplx_of<T>::type (&a)[NP]) {
+    const int i = RegGroup<NP>::lane();
+    T s = (T)0;
+#pragma unroll
+    for (int j = 0; j < NP; ++j) s += j == i ? (T)0 : a[j].x * a[j].x + a[j].y * a[j].y;
+    return RegGroup<NP>::sum(i < NP ? s : (T)0);
+}
+
+// Shared memory of one group: S matrices of NP rows of LD complex entries (16-byte rows), rotations.
+template <typename T, int NP, int S> struct RegSmem {
+    typedef typename cplx_of<T>::type C;
+    static constexpr int LD = NP + 2;
+    C m[S][NP * LD];
+    RegRot<T> rot[NP];
+};
+
+// Upper triangle of a stored Hermitian matrix into shared rows S[i * LD + j] (lower = conjugate, real
+// diagonal, zeros beyond nw); valid = 0 stores zeros.  Closes with __syncwarp.
+template <typename T, int NP>
+WNLQG_D void reg_stage_hermitian(typename cplx_of<T>::type *S, const double2 *__restrict__ h, int nw, bool valid) {
+    typedef typename cplx_of<T>::type C;
+    constexpr int LD = NP + 2;
+    const int i = RegGroup<NP>::lane();
+    if (i < NP)
+#pragma unroll 4
+        for (int j = 0; j < NP; ++j) {
+            if (j < i) continue;
+            double2 x = make_double2(0.0, 0.0);
+            if (valid && i < nw && j < nw) x = h[i + (int64_t)nw * j];
+            if (i == j) x.y = 0.0;
+            const C z = from_c64<C>(x);
+            S[i * LD + j] = z;
+            if (i != j) S[j * LD + i] = cconj(z);
+        }
+    __syncwarp();
+}
+
+// FP32 preconditioner of the orthogonal eigensolver (the first stage of eigh.cuh's two-stage scheme):
+// parallel Jacobi until the off-diagonal norm is below 2^-17 ||H|| (rotating elements above
+// 2^-20 ||H||), warm-started along runs of neighbouring points: V <- V (3I - V^H V) / 2,
+// A <- V^H H V.  Chain g of `chains` takes the points [batch g / chains, batch (g + 1) / chains).
+// Blocks of 128 threads.  A converged group of a warp is held (no element exceeds its tolerance)
+// until the warp's last group has converged (all lanes take every shuffle).
+// Bound by instruction issue (about 26 np per lane and round) with two warps per scheduler, as many
+// as the two matrices' 128 registers per lane allow.
+template <int NP>
+__global__ void __launch_bounds__(128, 2) jacobi_f32_reg_kernel(
+    const double2 *__restrict__ h_in, int64_t h_stride, int64_t batch, int nw, float2 *__restrict__ V_out,
+    int64_t chains, int warm_start) {
+    typedef RegGroup<NP> G;
+    typedef RegSmem<float, NP, 2> Smem;
+    constexpr int LD = Smem::LD;
+    extern __shared__ __align__(16) unsigned char reg_smem_raw[];
+    Smem &sm = reinterpret_cast<Smem *>(reg_smem_raw)[threadIdx.x / G::LANES];
+    float2 *S1 = sm.m[0], *S2 = sm.m[1];
+    const int i = G::lane(), ic = min(i, NP - 1);
+    const int64_t g = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / G::LANES;
+    const int64_t kb = g < chains ? (batch * g) / chains : 0, ke = g < chains ? (batch * (g + 1)) / chains : 0;
+    const int64_t steps = (batch + chains - 1) / chains;   // the longest chain: every group of a warp takes as many
+    float2 a[NP], v[NP];
+    auto row_to = [&](float2 *S, const float2(&x)[NP]) {
+        if (i < NP)
+#pragma unroll
+            for (int j = 0; j < NP; j += 2)
+                *reinterpret_cast<float4 *>(S + i * LD + j) = make_float4(x[j].x, x[j].y, x[j + 1].x, x[j + 1].y);
+    };
+    auto row_from = [&](const float2 *S, float2(&x)[NP]) {
+#pragma unroll
+        for (int j = 0; j < NP; j += 2) {
+            const float4 q = *reinterpret_cast<const float4 *>(S + ic * LD + j);
+            x[j] = make_float2(q.x, q.y);
+            x[j + 1] = make_float2(q.z, q.w);
+        }
+    };
+    // x[j] = sum_l f(l) Y[l][j], Y rows in shared memory.
+    auto product = [&](auto f, const float2 *Y, float2(&x)[NP]) {
+#pragma unroll
+        for (int j = 0; j < NP; ++j) x[j] = make_float2(0.0f, 0.0f);
+#pragma unroll 1
+        for (int l = 0; l < NP; ++l) {
+            const float2 w = f(l);
+#pragma unroll
+            for (int j = 0; j < NP; j += 2) {
+                const float4 y = *reinterpret_cast<const float4 *>(Y + l * LD + j);
+                x[j] = cfma(w, make_float2(y.x, y.y), x[j]);
+                x[j + 1] = cfma(w, make_float2(y.z, y.w), x[j + 1]);
+            }
+        }
+    };
+    for (int64_t step = 0; step < steps; ++step) {
+        const int64_t b = kb + step;
+        const bool valid = b < ke;
+        const double2 *h = h_in + (valid ? b : 0) * h_stride;
+        const bool warm = warm_start && step > 0;   // uniform over the warp
+        if (warm) {
+            row_to(S1, v);
+            __syncwarp();
+            product([&](int l) { return cconj(S1[l * LD + ic]); }, S1, a);            // V^H V
+#pragma unroll
+            for (int j = 0; j < NP; ++j) a[j] = make_float2((j == i ? 1.5f : 0.0f) - 0.5f * a[j].x, -0.5f * a[j].y);
+            row_to(S2, a);
+            __syncwarp();
+            product([&](int l) { return S1[ic * LD + l]; }, S2, v);                   // V M
+            __syncwarp();
+            row_to(S1, v);
+        }
+        reg_stage_hermitian<float, NP>(S2, h, nw, valid);
+        row_from(S2, a);
+        double f2 = 0.0;
+#pragma unroll
+        for (int j = 0; j < NP; ++j) f2 += (double)a[j].x * a[j].x + (double)a[j].y * a[j].y;
+        const double fro = sqrt(G::sum(i < NP ? f2 : 0.0));
+        if (warm) {
+            product([&](int l) { return cconj(S2[l * LD + ic]); }, S1, a);            // H V (H Hermitian)
+            __syncwarp();
+            row_to(S2, a);
+            __syncwarp();
+            product([&](int l) { return cconj(S1[l * LD + ic]); }, S2, a);            // V^H H V
+        } else {
+#pragma unroll
+            for (int j = 0; j < NP; ++j) v[j] = make_float2(j == i ? 1.0f : 0.0f, 0.0f);
+        }
+        float d = 0.0f;
+#pragma unroll
+        for (int j = 0; j < NP; ++j)
+            if (j == i) d = a[j].x;
+        float tol = (float)(fro * 9.5367431640625e-07);
+        const double stop = fro * 7.62939453125e-06;
+        bool done = !valid;
+        for (int sweep = 0; sweep < 30; ++sweep) {
+            const double off = sqrt((double)reg_offdiag2<float, NP>(a));   // every lane takes the shuffles
+            done = done || off <= stop;
+            if (__all_sync(0xffffffffu, done)) break;
+            if (done) tol = 3.0e18f;   // above every element: nothing rotates
+            const bool any = reg_jacobi_sweep<float, NP>(a, v, d, tol, sm.rot);
+            done = done || !any;
+        }
+        if (valid && i < NP) {
+            float2 *vo = V_out + b * (int64_t)NP * NP;
+#pragma unroll
+            for (int j = 0; j < NP; ++j) vo[i + (int64_t)NP * j] = v[j];
+        }
+        __syncwarp();
+    }
+}
+
+// FP64 spectrum of orthogonal models up to 16 orbitals, FP64 Jacobi from the identity to the FP64 CTA
+// Jacobi's stopping rule (off-diagonal norm <= np 2^-60 ||H||, or a sweep with every |a_pq| <=
+// 2^-60 ||H||), ascending order and canonical phases (jacobi_eigh_kernel).  Group g of the grid takes
+// the points g, g + groups, ...; no point depends on another, so nothing is gained by ordering them.
+// Blocks of 128 threads.  One kernel in place of an FP32 stage and an FP64 refinement of one warp per
+// matrix: 4 orbitals on a 32^3 mesh, the whole call 1.66 -> 0.56 ms (1.15 of it the two stages);
+// 33 points, 187 -> 140 us with the ordering that is no longer needed.
+template <int NP>
+__global__ void __launch_bounds__(128, NP > 8 ? 2 : 3) jacobi_f64_reg_kernel(
+    const double2 *__restrict__ h_in, int64_t h_stride, int64_t batch, int nw, double *__restrict__ E_out,
+    double2 *__restrict__ U_out) {
+    typedef RegGroup<NP> G;
+    typedef RegSmem<double, NP, 1> Smem;
+    constexpr int LD = Smem::LD;
+    extern __shared__ __align__(16) unsigned char reg_smem_raw[];
+    Smem &sm = reinterpret_cast<Smem *>(reg_smem_raw)[threadIdx.x / G::LANES];
+    double2 *S = sm.m[0];
+    const int i = G::lane(), ic = min(i, NP - 1);
+    const int64_t groups = (int64_t)gridDim.x * blockDim.x / G::LANES;
+    const int64_t g = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / G::LANES;
+    double2 a[NP], v[NP];
+    for (int64_t b0 = g - G::group(); b0 < batch; b0 += groups) {   // uniform over the warp
+        const int64_t b = b0 + G::group();
+        const bool valid = b < batch;
+        reg_stage_hermitian<double, NP>(S, h_in + (valid ? b : 0) * h_stride, nw, valid);
+        double f2 = 0.0, d = 0.0;
+#pragma unroll
+        for (int j = 0; j < NP; ++j) {
+            a[j] = S[ic * LD + j];
+            f2 += a[j].x * a[j].x + a[j].y * a[j].y;
+            if (j == i) d = a[j].x;
+            v[j] = make_double2(j == i ? 1.0 : 0.0, 0.0);
+        }
+        const double fro = sqrt(G::sum(i < NP ? f2 : 0.0));
+        double tol = fro * 8.673617379884035e-19;
+        const double stop = tol * NP;
+        bool done = !valid;
+        for (int sweep = 0; sweep < 30; ++sweep) {
+            const double off = sqrt(reg_offdiag2<double, NP>(a));   // every lane takes the shuffles
+            done = done || off <= stop;
+            if (__all_sync(0xffffffffu, done)) break;
+            if (done) tol = 1.0e150;   // nothing rotates
+            const bool any = reg_jacobi_sweep<double, NP>(a, v, d, tol, sm.rot);
+            done = done || !any;
+        }
+        // Lane i: rank of eigenvalue i (ascending, ties in index order), pivot and phase of its column.
+        int rank = 0;
+#pragma unroll
+        for (int j = 0; j < NP; ++j) {
+            const double dj = G::from(d, j);
+            if (j < nw) rank += (dj < d) || (dj == d && j < i);
+        }
+        __syncwarp();
+        if (i < NP)
+#pragma unroll
+            for (int j = 0; j < NP; ++j) S[i * LD + j] = v[j];
+        __syncwarp();
+        double2 phase = make_double2(1.0, 0.0);
+        {
+            int pivot = 0;
+            double pm = hypot(S[ic].x, S[ic].y);
+            for (int r = 1; r < nw; ++r) {
+                const double mg = hypot(S[r * LD + ic].x, S[r * LD + ic].y);
+                if (mg > pm) { pm = mg; pivot = r; }
+            }
+            if (pm > 0.0) phase = make_double2(S[pivot * LD + ic].x / pm, -S[pivot * LD + ic].y / pm);
+        }
+        if (valid && i < nw) E_out[b * nw + rank] = d;
+        double2 *u = U_out + (valid ? b : 0) * (int64_t)nw * nw;
+#pragma unroll
+        for (int j = 0; j < NP; ++j) {
+            const int rj = G::from(rank, j);
+            const double2 pj = make_double2(G::from(phase.x, j), G::from(phase.y, j));
+            if (valid && i < nw && j < nw) u[i + (int64_t)nw * rj] = cmul(v[j], pj);
+        }
+        __syncwarp();
+    }
+}
+
+// Kernel and group shared memory of an even order np.
+struct RegKernel {
+    const void *fn;
+    size_t group_smem;
+    int lanes;
+};
+template <int NP> RegKernel reg_f32_entry() {
+    return {(const void *)jacobi_f32_reg_kernel<NP>, sizeof(RegSmem<float, NP, 2>), RegGroup<NP>::LANES};
+}
+template <int NP> RegKernel reg_f64_entry() {
+    return {(const void *)jacobi_f64_reg_kernel<NP>, sizeof(RegSmem<double, NP, 1>), RegGroup<NP>::LANES};
+}
+inline RegKernel reg_f32_kernel(int np) {   // 18 <= np <= 32
+    static const RegKernel k[8] = {reg_f32_entry<18>(), reg_f32_entry<20>(), reg_f32_entry<22>(), reg_f32_entry<24>(),
+                                   reg_f32_entry<26>(), reg_f32_entry<28>(), reg_f32_entry<30>(), reg_f32_entry<32>()};
+    return k[(np - 18) / 2];
+}
+inline RegKernel reg_f64_kernel(int np) {
+    static const RegKernel k[8] = {reg_f64_entry<2>(),  reg_f64_entry<4>(),  reg_f64_entry<6>(),  reg_f64_entry<8>(),
+                                   reg_f64_entry<10>(), reg_f64_entry<12>(), reg_f64_entry<14>(), reg_f64_entry<16>()};
+    return k[np / 2 - 1];
+}

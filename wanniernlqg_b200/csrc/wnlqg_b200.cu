@@ -21,6 +21,7 @@
 
 #include "common.cuh"
 #include "eigh.cuh"
+#include "regjacobi.cuh"
 #include "fourier.cuh"
 #include "response.cuh"
 #include "shg.cuh"
@@ -150,7 +151,9 @@ struct wnlqg_plan {
     int eigh_threads = 32;
     size_t eigh_smem = 0;
     bool warp_eigh = false;                   // orthogonal models, nw <= 32: team-per-matrix stages
-    int eigh_team = 32;                       // threads per matrix in those stages: 32, 64 or 128
+    int eigh_team = 32;                       // threads per matrix of the FP64 refinement: 32, 64 or 128
+    bool f32_team = false;                    // first stage in shared memory (mixed path)
+    bool small_f64 = false;                   // FP64 path, nw <= 16: FP64 Jacobi in registers, no stages
     // Convention I: Cartesian and fractional Wannier centres (tau[a * nw + i]).
     bool conv1 = false;
     std::vector<double> tau_cart, tau_frac;
@@ -844,26 +847,58 @@ wnlqg_status setup_tc_fourier(wnlqg_plan *pl, const std::vector<double2> &tiles)
 // eigenvalues into d_E, canonical eigenvectors into d_U.  warm_in: warm-start along the batch.
 wnlqg_status run_orth_eigen(wnlqg_plan *pl, const double2 *hk, int64_t stride_in, int64_t nb, int warm_in) {
     if (pl->warp_eigh) {
-        // Stage 1: four one-warp teams per 128-thread block, or one 64-thread team per block.
+        const int np = pl->nw + (pl->nw & 1);
+        if (pl->small_f64) {
+            const RegKernel rk = reg_f64_kernel(np);
+            const int per_block = 128 / rk.lanes;
+            const size_t smem = rk.group_smem * per_block;
+            int per_sm = 1;
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, rk.fn, 128, smem);
+            const int64_t grid = std::min<int64_t>((nb + per_block - 1) / per_block, (int64_t)std::max(1, per_sm) * pl->sm_count);
+            int64_t stride = stride_in, nb_arg = nb;
+            int nw_arg = pl->nw;
+            double *E = pl->d_E;
+            double2 *U = pl->d_U;
+            void *args[] = {(void *)&hk, &stride, &nb_arg, &nw_arg, &E, &U};
+            WNLQG_CUDA(cudaLaunchKernel(rk.fn, dim3((unsigned)grid), dim3(128), args, smem, pl->stream));
+            WNLQG_CUDA(cudaGetLastError());
+            return WNLQG_OK;
+        }
+        // Stage 1, FP64 path (17 to 32 orbitals): one warp per chain of neighbouring points, eight
+        // chains per SM (what the kernel's registers hold).  32 orbitals, 32768 points of a 256^3
+        // mesh: 6.9 ms with the matrix in shared memory, 5.0 in registers.  The mixed path keeps the
+        // shared-memory stage: its one first-order completion leaves errors of second order in what
+        // stage 1 leaves, so the order of stage 1's roundings shows in its sums (up to 2e-8 relative).
         // Stage 2: 64-thread blocks holding two one-warp teams or one 64-thread team.
         const int tm = pl->eigh_team;
-        const void *f32_fn = tm == 128 ? (const void *)jacobi_f32_team_kernel<128>
-                             : tm == 64 ? (const void *)jacobi_f32_team_kernel<64> : (const void *)jacobi_f32_team_kernel<32>;
         const void *ref_fn = tm == 128 ? (const void *)eigh_refine_f64_team_kernel<128>
                              : tm == 64 ? (const void *)eigh_refine_f64_team_kernel<64> : (const void *)eigh_refine_f64_team_kernel<32>;
-        const int f32_threads = tm == 32 ? 128 : tm, f32_teams = tm == 32 ? 4 : 1;
         const int ref_threads = tm == 128 ? 128 : 64, ref_teams = tm == 32 ? 2 : 1;
-        int per_sm = 1;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, f32_fn, f32_threads, pl->eigh_smem);
-        const int64_t f32_grid = std::min<int64_t>((nb + f32_teams - 1) / f32_teams, (int64_t)std::max(1, per_sm) * pl->sm_count);
         int warm = warm_in;
-        {
+        if (pl->f32_team) {
+            const void *f32_fn = tm == 128 ? (const void *)jacobi_f32_team_kernel<128>
+                                 : tm == 64 ? (const void *)jacobi_f32_team_kernel<64> : (const void *)jacobi_f32_team_kernel<32>;
+            const int f32_threads = tm == 32 ? 128 : tm, f32_teams = tm == 32 ? 4 : 1;
+            int per_sm = 1;
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, f32_fn, f32_threads, pl->eigh_smem);
+            const int64_t f32_grid = std::min<int64_t>((nb + f32_teams - 1) / f32_teams, (int64_t)std::max(1, per_sm) * pl->sm_count);
             int64_t nb_arg = nb;
             int nw_arg = pl->nw;
             float2 *v32 = pl->d_V32;
             int64_t stride = stride_in;
             void *args[] = {(void *)&hk, &stride, &nb_arg, &nw_arg, &v32, &warm};
             WNLQG_CUDA(cudaLaunchKernel(f32_fn, dim3((unsigned)f32_grid), dim3(f32_threads), args, pl->eigh_smem, pl->stream));
+        } else {
+            const RegKernel rk = reg_f32_kernel(np);
+            const int per_block = 128 / rk.lanes;
+            int64_t chains = std::min<int64_t>(nb, (int64_t)8 * pl->sm_count);
+            int64_t nb_arg = nb;
+            int nw_arg = pl->nw;
+            float2 *v32 = pl->d_V32;
+            int64_t stride = stride_in;
+            void *args[] = {(void *)&hk, &stride, &nb_arg, &nw_arg, &v32, &chains, &warm};
+            WNLQG_CUDA(cudaLaunchKernel(rk.fn, dim3((unsigned)((chains + per_block - 1) / per_block)), dim3(128), args,
+                                        rk.group_smem * per_block, pl->stream));
         }
         int per_sm_r = 1;
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_r, ref_fn, ref_threads, pl->refine_smem);
@@ -1968,6 +2003,8 @@ wnlqg_status wnlqg_b200_plan_create(wnlqg_model *model, const wnlqg_task_desc *t
         pl->gen_mixed = pl->nonorth && t.precision == WNLQG_PRECISION_MIXED && !(gm && gm[0] == '0');
         const bool orth_stages = !pl->nonorth || pl->gen_mixed;
         pl->warp_eigh = orth_stages && nw <= 32 && !cta_fp64;
+        pl->f32_team = pl->warp_eigh && t.precision == WNLQG_PRECISION_MIXED;
+        pl->small_f64 = pl->warp_eigh && nw <= 16 && t.precision != WNLQG_PRECISION_MIXED;
         // Above 32 orbitals the CTA FP32 + FP64 stages; on the FP64 path only once two FP64 CTA
         // Jacobi working sets no longer fit one SM (there the plain FP64 Jacobi is faster).
         const bool fp64_cta_pair_fits =
@@ -1997,17 +2034,24 @@ wnlqg_status wnlqg_b200_plan_create(wnlqg_model *model, const wnlqg_task_desc *t
                 for (int k1 = 0; k1 < k2; ++k1, ++w) { off[w][0] = (unsigned char)k1; off[w][1] = (unsigned char)k2; }
             cudaError_t et = cudaMemcpyToSymbol(c_jacobi_offdiag, off, sizeof(off));
             if (et != cudaSuccess) return bail(fail(WNLQG_ERR_CUDA, std::string("cudaMemcpyToSymbol: ") + cudaGetErrorString(et)));
-            cudaError_t ea = allow_dynamic_smem((const void *)jacobi_f32_team_kernel<32>, smem_optin);
+            cudaError_t ea = cudaSuccess;
+            if (pl->small_f64) ea = allow_dynamic_smem(reg_f64_kernel(np).fn, smem_optin);
+            else if (!pl->f32_team) ea = allow_dynamic_smem(reg_f32_kernel(np).fn, smem_optin);
+            if (ea == cudaSuccess) ea = allow_dynamic_smem((const void *)jacobi_f32_team_kernel<32>, smem_optin);
             if (ea == cudaSuccess) ea = allow_dynamic_smem((const void *)jacobi_f32_team_kernel<64>, smem_optin);
             if (ea == cudaSuccess) ea = allow_dynamic_smem((const void *)jacobi_f32_team_kernel<128>, smem_optin);
+            if (ea == cudaSuccess && pl->small_f64) ea = allow_dynamic_smem(reg_f64_kernel(np).fn, smem_optin);
             if (ea != cudaSuccess) return bail(fail(WNLQG_ERR_CUDA, std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(ea)));
         }
         // Both stages need blockDim >= np/2 (pairs) and 8 * blockDim >= np^2 (register-staged products).
         pl->refine_threads = std::max(32, std::min(256, ((np * np / 8 + 31) / 32) * 32));
         pl->refine_threads = std::max(pl->refine_threads, ((np / 2 + 31) / 32) * 32);
         pl->eigh_threads = pl->refine_threads;
-        if ((st = alloc((void **)&pl->d_V32, (size_t)max_batch * np * np * sizeof(float2))) != WNLQG_OK) return bail(st);
-        if ((st = alloc_ordering()) != WNLQG_OK) return bail(st);
+        // Point ordering and the FP32 vectors serve the warm-started first stage.
+        if (!pl->small_f64) {
+            if ((st = alloc((void **)&pl->d_V32, (size_t)max_batch * np * np * sizeof(float2))) != WNLQG_OK) return bail(st);
+            if ((st = alloc_ordering()) != WNLQG_OK) return bail(st);
+        }
         cudaError_t e = allow_dynamic_smem((const void *)eigh_refine_f64_team_kernel<32>, smem_optin);
         if (e == cudaSuccess) e = allow_dynamic_smem((const void *)eigh_refine_f64_team_kernel<64>, smem_optin);
         if (e == cudaSuccess) e = allow_dynamic_smem((const void *)eigh_refine_f64_team_kernel<128>, smem_optin);
