@@ -1,7 +1,8 @@
-"""The register eigensolvers at their edges: every padded order up to 32 (odd counts, one orbital, the
-largest order of each group width, the FP64 kernel up to 16 and the FP32 stage from 17), fewer and
-more points than the groups of a warp and of the grid, and exactly degenerate levels, against the
-oracle's energies and the eigenvector residual."""
+"""The FP64 path's eigensolvers at their edges: every padded order up to 32 (odd counts, one orbital, the
+largest order of each group width, the register kernel up to 16 and the one-sided stage from 17), the
+CTA form's column blocks and rows per lane above 32, fewer and more points than the groups of a warp
+and of the grid, and exactly degenerate levels, against LAPACK's energies and the eigenvector
+residual."""
 import numpy as np
 import pytest
 
@@ -32,7 +33,8 @@ def check(model, k, vectors_for):
         assert np.max(np.abs(top.imag)) < 1e-12 and np.min(top.real) > 0
 
 
-@pytest.mark.parametrize("nw", [1, 2, 3, 4, 5, 7, 8, 9, 11, 13, 16, 17, 19, 22, 23, 26, 28, 29, 31, 32])
+@pytest.mark.parametrize("nw", [1, 2, 3, 4, 5, 7, 8, 9, 11, 13, 16, 17, 19, 22, 23, 26, 28, 29, 31, 32,
+                                33, 36, 37, 40, 41, 48, 63, 64, 65, 72, 95, 96, 97, 112, 128])
 def test_every_order(nw):
     model = synthetic_orthogonal_model(nw, 1, seed=100 + nw, full_position=True)
     check(model, np.random.default_rng(nw).random((7, 3)), range(7))
@@ -45,15 +47,16 @@ def test_point_counts(nw, points):
     check(model, np.random.default_rng(points).random((points, 3)), {0, points // 2, points - 1})
 
 
-@pytest.mark.parametrize("nw", [6, 14, 24])
+@pytest.mark.parametrize("nw", [6, 14, 24, 50])
 def test_degenerate_levels(nw):
     base = synthetic_orthogonal_model(nw // 2, 1, seed=3, full_position=True)
     check(kramers_doubled_model(base, 0.0), np.random.default_rng(5).random((6, 3)), range(6))
 
 
-def test_diagonal_and_zero_matrices():
-    ham = np.zeros((5, 5, 1), dtype=complex, order="F")
-    one = TightBindingModel(np.eye(3), np.zeros((3, 1), int), np.ones(1, int), ham, np.zeros((5, 5, 3, 1), complex))
-    check(one, np.zeros((2, 3)), range(2))
-    one.hamiltonian_r[:, :, 0] = np.diag([3.0, -1.0, 2.0, 2.0, 0.5])
+@pytest.mark.parametrize("nw", [5, 21, 39])
+@pytest.mark.parametrize("scale", [0.0, 1.0, 1e-9])
+def test_diagonal_and_zero_matrices(nw, scale):
+    ham = np.zeros((nw, nw, 1), dtype=complex, order="F")
+    one = TightBindingModel(np.eye(3), np.zeros((3, 1), int), np.ones(1, int), ham, np.zeros((nw, nw, 3, 1), complex))
+    one.hamiltonian_r[:, :, 0] = scale * np.diag(np.r_[3.0, -1.0, 2.0, 2.0, 0.5, np.linspace(-3.0, 1.0, nw - 5)])
     check(one, np.zeros((2, 3)), range(2))

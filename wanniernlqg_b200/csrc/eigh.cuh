@@ -240,8 +240,8 @@ __global__ void __launch_bounds__(256, 4) jacobi_eigh_kernel(const double2 *__re
 // Mixed-precision eigensolver up to 32 orbitals, in two kernels:
 //   stage 1: FP32 parallel Jacobi until the off-diagonal norm is below 2^-17 ||H||, warm-started
 //     along runs of consecutive mesh points from the previous point's eigenvectors (V <- V (3I -
-//     V^H V)/2, A <- V^H H V): on the FP64 path jacobi_f32_reg_kernel (regjacobi.cuh, the matrix in
-//     registers; up to 16 orbitals that path takes one FP64 kernel instead of the two stages), on the
+//     V^H V)/2, A <- V^H H V): on the FP64 path one-sided (onesided.cuh; up to 16
+//     orbitals that path takes one FP64 kernel, regjacobi.cuh, instead of the two stages), on the
 //     mixed path jacobi_f32_team_kernel (run_orth_eigen says why);
 //   stage 2 (eigh_refine_f64_team_kernel): FP64 Rayleigh-Ritz refinement by one team of TEAM threads
 //     per matrix, W = second-order Loewdin orthonormalisation of V, H' = W^H H W, FP64 Jacobi sweeps
@@ -1097,41 +1097,51 @@ __global__ void __launch_bounds__(512, 1) eigh_refine_f64_cta_kernel(const doubl
         dmma_product<0>(Wc, A, Tc, np, ld);                  // T = W M
         __syncthreads();
         { double2 *x = Wc; Wc = Tc; Tc = x; }                // W <- W M
-        // A <- H (Hermitian from the upper triangle, zero-padded), Frobenius norm.
+        // A <- W^H H W (exactly Hermitian), H from its upper triangle, zero-padded; returns ||H||_F.
         const double2 *h = h_in + b * h_stride;
-        double local = 0.0;
-        for (int e = tid; e < np * np; e += blockDim.x) {
-            const int i = e % np, j = e / np;
-            double2 v = make_double2(0.0, 0.0);
-            if (i < nw && j < nw) {
-                if (i < j) v = h[i + (size_t)nw * j];
-                else if (i > j) v = cconj(h[j + (size_t)nw * i]);
-                else v = make_double2(h[i + (size_t)nw * i].x, 0.0);
+        auto project = [&]() {
+            double local = 0.0;
+            for (int e = tid; e < np * np; e += blockDim.x) {
+                const int i = e % np, j = e / np;
+                double2 v = make_double2(0.0, 0.0);
+                if (i < nw && j < nw) {
+                    if (i < j) v = h[i + (size_t)nw * j];
+                    else if (i > j) v = cconj(h[j + (size_t)nw * i]);
+                    else v = make_double2(h[i + (size_t)nw * i].x, 0.0);
+                }
+                local += v.x * v.x + v.y * v.y;
+                A[i + ld * j] = v;
             }
-            local += v.x * v.x + v.y * v.y;
-            A[i + ld * j] = v;
-        }
-        for (int o = 16; o > 0; o >>= 1) local += __shfl_down_sync(0xffffffffu, local, o);
-        if ((tid & 31) == 0) red[tid >> 5] = local;
-        __syncthreads();
-        double fro = 0.0;
-        for (int w = 0; w < (int)(blockDim.x >> 5); ++w) fro += red[w];
-        fro = sqrt(fro);
-        dmma_product<0>(A, Wc, Tc, np, ld);                  // T = H W
-        __syncthreads();
-        dmma_product<1>(Wc, Tc, A, np, ld);                  // A = W^H H W
-        __syncthreads();
-        for (int e = tid; e < np * np; e += blockDim.x) {    // exact Hermitian symmetry
-            const int i = e % np, j = e / np;
-            if (i > j) A[i + ld * j] = cconj(A[j + ld * i]);
-            else if (i == j) A[i + ld * i].y = 0.0;
-        }
-        __syncthreads();
+            for (int o = 16; o > 0; o >>= 1) local += __shfl_down_sync(0xffffffffu, local, o);
+            if ((tid & 31) == 0) red[tid >> 5] = local;
+            __syncthreads();
+            double f = 0.0;
+            for (int w = 0; w < (int)(blockDim.x >> 5); ++w) f += red[w];
+            dmma_product<0>(A, Wc, Tc, np, ld);                  // T = H W
+            __syncthreads();
+            dmma_product<1>(Wc, Tc, A, np, ld);                  // A = W^H H W
+            __syncthreads();
+            for (int e = tid; e < np * np; e += blockDim.x) {    // exact Hermitian symmetry
+                const int i = e % np, j = e / np;
+                if (i > j) A[i + ld * j] = cconj(A[j + ld * i]);
+                else if (i == j) A[i + ld * i].y = 0.0;
+            }
+            __syncthreads();
+            return sqrt(f);
+        };
+        const double fro = project();
         const double tol = fro * 8.673617379884035e-19;
+        // FP64 path: the loose completion and a fresh projection before the strict one, as in the team
+        // kernel; the sweeps are the fallback of either bound.
+        bool loose = false;
+        if (converge && cta_first_order_completion(A, Wc, Tc, np, ld, reinterpret_cast<double *>(rot_s), 1.220703125e-04)) {
+            loose = true;
+            project();
+        }
         for (int sweep = 0; sweep < (converge ? WNLQG_JACOBI_MAX_SWEEPS : 1); ++sweep) {
             const double off = offdiag_norm(A, np, ld, red);
             if (off <= (converge ? tol * np : fro * 1.0e-13)) break;
-            if ((converge ? sweep > 0 : sweep == 0) &&
+            if ((converge ? (sweep > 0 || loose) : sweep == 0) &&
                 cta_first_order_completion(A, Wc, Tc, np, ld, reinterpret_cast<double *>(rot_s),
                                            converge ? 1.4901161193847656e-08 : 1.220703125e-04))
                 break;

@@ -1,5 +1,5 @@
-// regjacobi.cuh - Hermitian Jacobi with the matrix in registers: one group of lanes per matrix, lane i
-// holding row i of A and of the eigenvectors V, for orders up to 16 (FP64) and 18 to 32 (FP32).
+// regjacobi.cuh - FP64 Hermitian Jacobi with the matrix in registers, for orders up to 16: one group of
+// lanes per matrix, lane i holding row i of A and of the eigenvectors V.
 //
 // The rounds are those of the shared-memory sweeps (eigh.cuh): the circle method pairs the np indices
 // (np even), and A <- J^H A J, V <- V J per round.  Columns are kept in slots: slot 0 holds index 0,
@@ -13,7 +13,7 @@
 //   - the row rotations of A: each lane exchanges its row with its partner's by shuffles.
 // There is no barrier beyond __syncwarp, and shared memory carries the np / 2 rotations only; the
 // shared-memory form moved both matrices through it twice per round, with two block barriers.
-// Order np <= 16 puts two groups of 16 lanes (np <= 8: four of 8, np <= 4: eight of 4) in a warp.
+// A warp holds two groups of 16 lanes (np <= 8: four of 8, np <= 4: eight of 4).
 #pragma once
 #include "common.cuh"
 
@@ -188,115 +188,6 @@ WNLQG_D void reg_stage_hermitian(typename cplx_of<T>::type *S, const double2 *__
     __syncwarp();
 }
 
-// FP32 preconditioner of the orthogonal eigensolver (the first stage of eigh.cuh's two-stage scheme):
-// parallel Jacobi until the off-diagonal norm is below 2^-17 ||H|| (rotating elements above
-// 2^-20 ||H||), warm-started along runs of neighbouring points: V <- V (3I - V^H V) / 2,
-// A <- V^H H V.  Chain g of `chains` takes the points [batch g / chains, batch (g + 1) / chains).
-// Blocks of 128 threads.  A converged group of a warp is held (no element exceeds its tolerance)
-// until the warp's last group has converged (all lanes take every shuffle).
-// Bound by instruction issue (about 26 np per lane and round) with two warps per scheduler, as many
-// as the two matrices' 128 registers per lane allow.
-template <int NP>
-__global__ void __launch_bounds__(128, 2) jacobi_f32_reg_kernel(
-    const double2 *__restrict__ h_in, int64_t h_stride, int64_t batch, int nw, float2 *__restrict__ V_out,
-    int64_t chains, int warm_start) {
-    typedef RegGroup<NP> G;
-    typedef RegSmem<float, NP, 2> Smem;
-    constexpr int LD = Smem::LD;
-    extern __shared__ __align__(16) unsigned char reg_smem_raw[];
-    Smem &sm = reinterpret_cast<Smem *>(reg_smem_raw)[threadIdx.x / G::LANES];
-    float2 *S1 = sm.m[0], *S2 = sm.m[1];
-    const int i = G::lane(), ic = min(i, NP - 1);
-    const int64_t g = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / G::LANES;
-    const int64_t kb = g < chains ? (batch * g) / chains : 0, ke = g < chains ? (batch * (g + 1)) / chains : 0;
-    const int64_t steps = (batch + chains - 1) / chains;   // the longest chain: every group of a warp takes as many
-    float2 a[NP], v[NP];
-    auto row_to = [&](float2 *S, const float2(&x)[NP]) {
-        if (i < NP)
-#pragma unroll
-            for (int j = 0; j < NP; j += 2)
-                *reinterpret_cast<float4 *>(S + i * LD + j) = make_float4(x[j].x, x[j].y, x[j + 1].x, x[j + 1].y);
-    };
-    auto row_from = [&](const float2 *S, float2(&x)[NP]) {
-#pragma unroll
-        for (int j = 0; j < NP; j += 2) {
-            const float4 q = *reinterpret_cast<const float4 *>(S + ic * LD + j);
-            x[j] = make_float2(q.x, q.y);
-            x[j + 1] = make_float2(q.z, q.w);
-        }
-    };
-    // x[j] = sum_l f(l) Y[l][j], Y rows in shared memory.
-    auto product = [&](auto f, const float2 *Y, float2(&x)[NP]) {
-#pragma unroll
-        for (int j = 0; j < NP; ++j) x[j] = make_float2(0.0f, 0.0f);
-#pragma unroll 1
-        for (int l = 0; l < NP; ++l) {
-            const float2 w = f(l);
-#pragma unroll
-            for (int j = 0; j < NP; j += 2) {
-                const float4 y = *reinterpret_cast<const float4 *>(Y + l * LD + j);
-                x[j] = cfma(w, make_float2(y.x, y.y), x[j]);
-                x[j + 1] = cfma(w, make_float2(y.z, y.w), x[j + 1]);
-            }
-        }
-    };
-    for (int64_t step = 0; step < steps; ++step) {
-        const int64_t b = kb + step;
-        const bool valid = b < ke;
-        const double2 *h = h_in + (valid ? b : 0) * h_stride;
-        const bool warm = warm_start && step > 0;   // uniform over the warp
-        if (warm) {
-            row_to(S1, v);
-            __syncwarp();
-            product([&](int l) { return cconj(S1[l * LD + ic]); }, S1, a);            // V^H V
-#pragma unroll
-            for (int j = 0; j < NP; ++j) a[j] = make_float2((j == i ? 1.5f : 0.0f) - 0.5f * a[j].x, -0.5f * a[j].y);
-            row_to(S2, a);
-            __syncwarp();
-            product([&](int l) { return S1[ic * LD + l]; }, S2, v);                   // V M
-            __syncwarp();
-            row_to(S1, v);
-        }
-        reg_stage_hermitian<float, NP>(S2, h, nw, valid);
-        row_from(S2, a);
-        double f2 = 0.0;
-#pragma unroll
-        for (int j = 0; j < NP; ++j) f2 += (double)a[j].x * a[j].x + (double)a[j].y * a[j].y;
-        const double fro = sqrt(G::sum(i < NP ? f2 : 0.0));
-        if (warm) {
-            product([&](int l) { return cconj(S2[l * LD + ic]); }, S1, a);            // H V (H Hermitian)
-            __syncwarp();
-            row_to(S2, a);
-            __syncwarp();
-            product([&](int l) { return cconj(S1[l * LD + ic]); }, S2, a);            // V^H H V
-        } else {
-#pragma unroll
-            for (int j = 0; j < NP; ++j) v[j] = make_float2(j == i ? 1.0f : 0.0f, 0.0f);
-        }
-        float d = 0.0f;
-#pragma unroll
-        for (int j = 0; j < NP; ++j)
-            if (j == i) d = a[j].x;
-        float tol = (float)(fro * 9.5367431640625e-07);
-        const double stop = fro * 7.62939453125e-06;
-        bool done = !valid;
-        for (int sweep = 0; sweep < 30; ++sweep) {
-            const double off = sqrt((double)reg_offdiag2<float, NP>(a));   // every lane takes the shuffles
-            done = done || off <= stop;
-            if (__all_sync(0xffffffffu, done)) break;
-            if (done) tol = 3.0e18f;   // above every element: nothing rotates
-            const bool any = reg_jacobi_sweep<float, NP>(a, v, d, tol, sm.rot);
-            done = done || !any;
-        }
-        if (valid && i < NP) {
-            float2 *vo = V_out + b * (int64_t)NP * NP;
-#pragma unroll
-            for (int j = 0; j < NP; ++j) vo[i + (int64_t)NP * j] = v[j];
-        }
-        __syncwarp();
-    }
-}
-
 // FP64 spectrum of orthogonal models up to 16 orbitals, FP64 Jacobi from the identity to the FP64 CTA
 // Jacobi's stopping rule (off-diagonal norm <= np 2^-60 ||H||, or a sweep with every |a_pq| <=
 // 2^-60 ||H||), ascending order and canonical phases (jacobi_eigh_kernel).  Group g of the grid takes
@@ -382,16 +273,8 @@ struct RegKernel {
     size_t group_smem;
     int lanes;
 };
-template <int NP> RegKernel reg_f32_entry() {
-    return {(const void *)jacobi_f32_reg_kernel<NP>, sizeof(RegSmem<float, NP, 2>), RegGroup<NP>::LANES};
-}
 template <int NP> RegKernel reg_f64_entry() {
     return {(const void *)jacobi_f64_reg_kernel<NP>, sizeof(RegSmem<double, NP, 1>), RegGroup<NP>::LANES};
-}
-inline RegKernel reg_f32_kernel(int np) {   // 18 <= np <= 32
-    static const RegKernel k[8] = {reg_f32_entry<18>(), reg_f32_entry<20>(), reg_f32_entry<22>(), reg_f32_entry<24>(),
-                                   reg_f32_entry<26>(), reg_f32_entry<28>(), reg_f32_entry<30>(), reg_f32_entry<32>()};
-    return k[(np - 18) / 2];
 }
 inline RegKernel reg_f64_kernel(int np) {
     static const RegKernel k[8] = {reg_f64_entry<2>(),  reg_f64_entry<4>(),  reg_f64_entry<6>(),  reg_f64_entry<8>(),

@@ -22,6 +22,7 @@
 #include "common.cuh"
 #include "eigh.cuh"
 #include "regjacobi.cuh"
+#include "onesided.cuh"
 #include "fourier.cuh"
 #include "response.cuh"
 #include "shg.cuh"
@@ -199,8 +200,8 @@ struct wnlqg_plan {
     // FP64 response passes on the 512-thread variant (WNLQG_B200_RESPONSE_WIDE at plan creation,
     // then the autotuner).
     bool resp_wide = false;
-    // Nonorthogonal models on the mixed path: FP64 Cholesky reduction C = L^-1 H L^-H (d_gC, with
-    // L in d_gL), the orthogonal mixed-precision stages on C, back-substitution U = L^-H V.
+    // Nonorthogonal models: FP64 Cholesky reduction C = L^-1 H L^-H (d_gC, with L in d_gL), the
+    // orthogonal stages on C, back-substitution U = L^-H V.
     bool gen_mixed = false;
     double2 *d_gC = nullptr, *d_gL = nullptr;
     size_t gred_smem = 0;
@@ -864,11 +865,10 @@ wnlqg_status run_orth_eigen(wnlqg_plan *pl, const double2 *hk, int64_t stride_in
             WNLQG_CUDA(cudaGetLastError());
             return WNLQG_OK;
         }
-        // Stage 1, FP64 path (17 to 32 orbitals): one warp per chain of neighbouring points, eight
-        // chains per SM (what the kernel's registers hold).  32 orbitals, 32768 points of a 256^3
-        // mesh: 6.9 ms with the matrix in shared memory, 5.0 in registers.  The mixed path keeps the
-        // shared-memory stage: its one first-order completion leaves errors of second order in what
-        // stage 1 leaves, so the order of stage 1's roundings shows in its sums (up to 2e-8 relative).
+        // Stage 1, FP64 path (17 to 32 orbitals): one-sided Jacobi, one warp per chain of neighbouring
+        // points, twelve chains per SM (what the kernel's registers hold).  The mixed path keeps the
+        // two-sided stage in shared memory: its one first-order completion leaves errors of second
+        // order in what stage 1 leaves, so another stage 1 would show in its sums (2e-8 relative).
         // Stage 2: 64-thread blocks holding two one-warp teams or one 64-thread team.
         const int tm = pl->eigh_team;
         const void *ref_fn = tm == 128 ? (const void *)eigh_refine_f64_team_kernel<128>
@@ -889,9 +889,9 @@ wnlqg_status run_orth_eigen(wnlqg_plan *pl, const double2 *hk, int64_t stride_in
             void *args[] = {(void *)&hk, &stride, &nb_arg, &nw_arg, &v32, &warm};
             WNLQG_CUDA(cudaLaunchKernel(f32_fn, dim3((unsigned)f32_grid), dim3(f32_threads), args, pl->eigh_smem, pl->stream));
         } else {
-            const RegKernel rk = reg_f32_kernel(np);
+            const RegKernel rk = onesided_kernel(np);
             const int per_block = 128 / rk.lanes;
-            int64_t chains = std::min<int64_t>(nb, (int64_t)8 * pl->sm_count);
+            int64_t chains = std::min<int64_t>(nb, (int64_t)12 * pl->sm_count);
             int64_t nb_arg = nb;
             int nw_arg = pl->nw;
             float2 *v32 = pl->d_V32;
@@ -918,7 +918,18 @@ wnlqg_status run_orth_eigen(wnlqg_plan *pl, const double2 *hk, int64_t stride_in
         const int converge = pl->task.precision == WNLQG_PRECISION_MIXED ? 0 : 1;
         const int warm = warm_in;
         const int64_t N = stride_in;
-        if (pl->cta_gw1) {
+        if (converge) {
+            const void *fn = onesided_cta_fn(pl->nw + (pl->nw & 1));
+            const int threads = OsCtaSmem::threads(pl->nw + (pl->nw & 1));
+            int per_sm = 1;
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, threads, pl->eigh_smem);
+            const int64_t grid = std::min<int64_t>(nb, (int64_t)std::max(1, per_sm) * pl->sm_count);
+            int64_t stride = N, nb_arg = nb;
+            int nw_arg = pl->nw, warm_arg = warm;
+            float2 *v32 = pl->d_V32;
+            void *args[] = {(void *)&hk, &stride, &nb_arg, &nw_arg, &v32, &warm_arg};
+            WNLQG_CUDA(cudaLaunchKernel(fn, dim3((unsigned)grid), dim3(threads), args, pl->eigh_smem, pl->stream));
+        } else if (pl->cta_gw1) {
             jacobi_f32_cta_kernel<true><<<(unsigned)std::min<int64_t>(nb, pl->eigh_grid), 256, 0, pl->stream>>>(
                 hk, N, nb, pl->nw, pl->d_V32, pl->d_eigh_scratch, pl->eigh_scratch_stride, warm);
         } else {
@@ -1737,7 +1748,7 @@ wnlqg_status wnlqg_b200_plan_create(wnlqg_model *model, const wnlqg_task_desc *t
     if (max_batch <= 0) {
         int64_t per_k = (int64_t)pl->C * nn * 16 + (int64_t)nr * 16 + nn * 16 + nw * 8 + vc * 16;
         if (pl->metric_shg) per_k += MetricShgWs::src_entries(nw) * 16 + MetricShgWs::diag_entries(nw) * 8;
-        if (pl->nonorth && t.precision == WNLQG_PRECISION_MIXED) per_k += 2 * nn * 16 + nn * 8;
+        if (pl->nonorth) per_k += 2 * nn * 16 + nn * 8;
         per_k += (int64_t)2 * pl->fd_nd * pl->fd_npair * nw * 8 + (pl->fd_nd > 0 ? 24 : 0);
         // About 4 GiB of batch workspace (HBM is 180 GB): long runs of neighbouring k-points per
         // CTA for the warm-started eigensolver and few batches per call.
@@ -1996,21 +2007,18 @@ wnlqg_status wnlqg_b200_plan_create(wnlqg_model *model, const wnlqg_task_desc *t
     {
         const char *cta = std::getenv("WNLQG_B200_CTA_EIGH");
         const bool cta_fp64 = cta && cta[0] == '1' && t.precision != WNLQG_PRECISION_MIXED;
-        // Nonorthogonal models on the mixed path reduce to C = L^-1 H L^-H in FP64 and then take
-        // the orthogonal mixed-precision stages (WNLQG_B200_GEN_MIXED=0 keeps the FP64 generalised
-        // Jacobi).
+        // Nonorthogonal models reduce to C = L^-1 H L^-H in FP64 and then take the orthogonal stages of
+        // their precision (WNLQG_B200_GEN_MIXED=0, and WNLQG_B200_CTA_EIGH=1 on the FP64 path, keep the
+        // FP64 generalised Jacobi: 64 orbitals, 1024 points, 14.0 ms against 4.8 for
+        // the four kernels).
         const char *gm = std::getenv("WNLQG_B200_GEN_MIXED");
-        pl->gen_mixed = pl->nonorth && t.precision == WNLQG_PRECISION_MIXED && !(gm && gm[0] == '0');
+        pl->gen_mixed = pl->nonorth && !cta_fp64 && !(gm && gm[0] == '0');
         const bool orth_stages = !pl->nonorth || pl->gen_mixed;
         pl->warp_eigh = orth_stages && nw <= 32 && !cta_fp64;
         pl->f32_team = pl->warp_eigh && t.precision == WNLQG_PRECISION_MIXED;
         pl->small_f64 = pl->warp_eigh && nw <= 16 && t.precision != WNLQG_PRECISION_MIXED;
-        // Above 32 orbitals the CTA FP32 + FP64 stages; on the FP64 path only once two FP64 CTA
-        // Jacobi working sets no longer fit one SM (there the plain FP64 Jacobi is faster).
-        const bool fp64_cta_pair_fits =
-            2 * (EighSmem::bytes(nw, sizeof(double2)) + 512) <= (size_t)smem_optin;
-        pl->cta_mixed = orth_stages && nw > 32 && !cta_fp64 &&
-                        (t.precision == WNLQG_PRECISION_MIXED || !fp64_cta_pair_fits);
+        // Above 32 orbitals the CTA stages: FP32 one-sided (mixed path: two-sided) and FP64 refinement.
+        pl->cta_mixed = orth_stages && nw > 32 && !cta_fp64;
     }
     if (pl->nonorth && !pl->gen_mixed) {
         pl->eigh_threads = std::max(pl->eigh_threads, ((nw + (nw & 1)) / 2 + 31) / 32 * 32);
@@ -2036,7 +2044,7 @@ wnlqg_status wnlqg_b200_plan_create(wnlqg_model *model, const wnlqg_task_desc *t
             if (et != cudaSuccess) return bail(fail(WNLQG_ERR_CUDA, std::string("cudaMemcpyToSymbol: ") + cudaGetErrorString(et)));
             cudaError_t ea = cudaSuccess;
             if (pl->small_f64) ea = allow_dynamic_smem(reg_f64_kernel(np).fn, smem_optin);
-            else if (!pl->f32_team) ea = allow_dynamic_smem(reg_f32_kernel(np).fn, smem_optin);
+            else if (!pl->f32_team) ea = allow_dynamic_smem(onesided_kernel(np).fn, smem_optin);
             if (ea == cudaSuccess) ea = allow_dynamic_smem((const void *)jacobi_f32_team_kernel<32>, smem_optin);
             if (ea == cudaSuccess) ea = allow_dynamic_smem((const void *)jacobi_f32_team_kernel<64>, smem_optin);
             if (ea == cudaSuccess) ea = allow_dynamic_smem((const void *)jacobi_f32_team_kernel<128>, smem_optin);
@@ -2068,6 +2076,10 @@ wnlqg_status wnlqg_b200_plan_create(wnlqg_model *model, const wnlqg_task_desc *t
         if (fe == cudaSuccess) fe = cudaFuncGetAttributes(&fa2, (const void *)eigh_refine_f64_cta_kernel<false>);
         if (fe != cudaSuccess) return bail(fail(WNLQG_ERR_CUDA, std::string("cudaFuncGetAttributes: ") + cudaGetErrorString(fe)));
         pl->cta_gw1 = pl->eigh_smem + fa1.sharedSizeBytes > (size_t)smem_optin;
+        if (t.precision != WNLQG_PRECISION_MIXED) {
+            pl->cta_gw1 = false;   // the one-sided stage always fits shared memory
+            pl->eigh_smem = OsCtaSmem::bytes(np);
+        }
         pl->cta_gw2 = pl->refine_smem + fa2.sharedSizeBytes > (size_t)smem_optin;
         // 256-thread refinement blocks when two fit an SM (shared memory and registers), else 512.
         pl->refine_cta_threads =
@@ -2085,7 +2097,8 @@ wnlqg_status wnlqg_b200_plan_create(wnlqg_model *model, const wnlqg_task_desc *t
                 return bail(st);
         }
         cudaError_t e = cudaSuccess;
-        if (!pl->cta_gw1) e = allow_dynamic_smem((const void *)jacobi_f32_cta_kernel<false>, smem_optin);
+        if (t.precision != WNLQG_PRECISION_MIXED) e = allow_dynamic_smem(onesided_cta_fn(np), smem_optin);
+        else if (!pl->cta_gw1) e = allow_dynamic_smem((const void *)jacobi_f32_cta_kernel<false>, smem_optin);
         if (e == cudaSuccess && !pl->cta_gw2) e = allow_dynamic_smem((const void *)eigh_refine_f64_cta_kernel<false>, smem_optin);
         if (e != cudaSuccess) return bail(fail(WNLQG_ERR_CUDA, std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(e)));
     } else {
