@@ -259,6 +259,11 @@ WNLQG_API wnlqg_status wnlqg_b200_eval_mesh_weighted(wnlqg_plan *plan, const int
 WNLQG_API wnlqg_status wnlqg_b200_eval_spectrum(wnlqg_plan *plan, const double *kpoints, int64_t n,
                                       double *energies, double *eigenvectors);
 
+/* The same with each point's eigenvectors in row-major order (row i, band n at i * nw + n), for callers
+ * whose arrays are row-major; the transposition runs on the device.  Convention II. */
+WNLQG_API wnlqg_status wnlqg_b200_eval_spectrum_rows(wnlqg_plan *plan, const double *kpoints, int64_t n,
+                                           double *energies, double *eigenvectors);
+
 /* Allocation-free spectrum (no counterpart in the reference).  For callers that cannot let this
  * library allocate device memory (their memory belongs to another pool allocator under a fixed
  * budget).  Inputs and outputs are caller-owned DEVICE arrays on the current device:

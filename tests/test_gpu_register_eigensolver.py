@@ -60,3 +60,21 @@ def test_diagonal_and_zero_matrices(nw, scale):
     one = TightBindingModel(np.eye(3), np.zeros((3, 1), int), np.ones(1, int), ham, np.zeros((nw, nw, 3, 1), complex))
     one.hamiltonian_r[:, :, 0] = scale * np.diag(np.r_[3.0, -1.0, 2.0, 2.0, 0.5, np.linspace(-3.0, 1.0, nw - 5)])
     check(one, np.zeros((2, 3)), range(2))
+
+
+@pytest.mark.parametrize("nw,points", [(3, 5), (13, 2001), (33, 801)])
+def test_row_and_column_major_vectors(nw, points):
+    """The row-major spectrum (device transposition, pinned chunks: none, several with a remainder, a
+    batch boundary inside) is the column-major one transposed, bit for bit."""
+    import ctypes
+    from wanniernlqg_b200.engine import ResponseEngine
+    model = synthetic_orthogonal_model(nw, 1, seed=nw)
+    k = np.random.default_rng(nw).random((points, 3))
+    dp = ctypes.POINTER(ctypes.c_double)
+    with ResponseEngine(model, _abi.TaskArrays([(_abi.QUANTUM_METRIC, ["xx"])]), max_batch=700) as eng:
+        e, u = eng.spectrum(k)
+        ec, uc = np.zeros_like(e), np.zeros((points, nw, nw), dtype=np.complex128)
+        assert eng._L.wnlqg_b200_eval_spectrum(eng._plan, k.ctypes.data_as(dp), points, ec.ctypes.data_as(dp),
+                                               uc.ctypes.data_as(dp)) == 0
+    assert np.array_equal(e, ec) and np.array_equal(u, uc.transpose(0, 2, 1))
+    assert u.flags["C_CONTIGUOUS"]

@@ -19,7 +19,7 @@ EXPORTED_SYMBOLS = (
     "wnlqg_b200_plan_create", "wnlqg_b200_plan_destroy", "wnlqg_b200_plan_value_count",
     "wnlqg_b200_eval_mesh", "wnlqg_b200_eval_mesh_device", "wnlqg_b200_eval_mesh_many", "wnlqg_b200_eval_points",
     "wnlqg_b200_eval_points_weighted", "wnlqg_b200_eval_points_weighted_device", "wnlqg_b200_eval_mesh_weighted",
-    "wnlqg_b200_eval_spectrum", "wnlqg_b200_plan_last_timing", "wnlqg_b200_plan_last_launch_count",
+    "wnlqg_b200_eval_spectrum", "wnlqg_b200_eval_spectrum_rows", "wnlqg_b200_plan_last_timing", "wnlqg_b200_plan_last_launch_count",
     "wnlqg_b200_spectrum_noalloc",
     "wnlqg_b200_mlp_param_count", "wnlqg_b200_mlp_create", "wnlqg_b200_mlp_destroy", "wnlqg_b200_mlp_get_params",
     "wnlqg_b200_mlp_set_params", "wnlqg_b200_mlp_forward", "wnlqg_b200_mlp_loss_grad", "wnlqg_b200_mlp_train",
@@ -69,6 +69,7 @@ def load():
     L.wnlqg_b200_eval_points_weighted_device.argtypes = [vp, vp, vp, ctypes.c_int64, vp, vp]
     L.wnlqg_b200_eval_mesh_weighted.argtypes = [vp, ip, ip, dp, ctypes.c_int64, dp]
     L.wnlqg_b200_eval_spectrum.argtypes = [vp, dp, ctypes.c_int64, dp, dp]
+    L.wnlqg_b200_eval_spectrum_rows.argtypes = [vp, dp, ctypes.c_int64, dp, dp]
     L.wnlqg_b200_plan_last_timing.argtypes = [vp, dp, dp, dp, dp]
     L.wnlqg_b200_spectrum_noalloc.argtypes = [ctypes.c_int64, ctypes.c_int64, vp, vp, vp, vp, ctypes.c_int64, vp, vp,
                                               vp]
@@ -112,6 +113,7 @@ def load():
                  "wnlqg_b200_eval_mesh_device", "wnlqg_b200_eval_mesh_many", "wnlqg_b200_eval_points",
                  "wnlqg_b200_eval_points_weighted",
                  "wnlqg_b200_eval_points_weighted_device", "wnlqg_b200_eval_mesh_weighted", "wnlqg_b200_eval_spectrum",
+                 "wnlqg_b200_eval_spectrum_rows",
                  "wnlqg_b200_plan_last_timing"):
         getattr(L, name).restype = ctypes.c_int
     _lib = L

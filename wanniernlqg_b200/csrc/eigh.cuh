@@ -858,16 +858,17 @@ __global__ void __launch_bounds__(TEAM == 128 ? 128 : 64, TEAM == 32 ? 1 : (TEAM
 // ---------------------------------------------------------------------------------------------
 // Mixed-precision eigensolver above 32 orbitals, one CTA per matrix, in two kernels (the same
 // scheme as the team kernels, for matrices a warp team cannot hold):
-//   stage 1 (jacobi_f32_cta_kernel): FP32 parallel Jacobi until the off-diagonal norm is below
-//     2^-17 ||H|| (rotating elements above 2^-20 ||H||), eigenvectors written unsorted; each CTA
-//     takes a contiguous range of points and, along mesh runs and Morton-ordered point batches,
-//     warm-starts each point from the previous one's eigenvectors;
+//   stage 1: on the FP64 path one-sided (onesided_cta_kernel, onesided.cuh); on the mixed path
+//     jacobi_f32_cta_kernel, FP32 parallel Jacobi until the off-diagonal norm is below 2^-17 ||H||
+//     (rotating elements above 2^-20 ||H||), eigenvectors written unsorted; each CTA takes a
+//     contiguous range of points and, along mesh runs and Morton-ordered point batches, warm-starts
+//     each point from the previous one's eigenvectors;
 //   stage 2 (eigh_refine_f64_cta_kernel): W = second-order Loewdin orthonormalisation of V
-//     (E = W^H W - I, W <- W (I - E/2 + 3E^2/8)), H' = W^H H W, FP64 Jacobi sweeps (mixed path:
-//     one, unless H' is diagonal to 1e-13 ||H||; FP64 path: until the FP64 CTA Jacobi's stopping
-//     rule holds, np 2^-60 ||H||, from the second sweep on replaced by the first-order completion
-//     when its bound holds), U = W J, ascending order and canonical phases.  The products run on
-//     the FP64 tensor cores (dmma_product).
+//     (E = W^H W - I, W <- W (I - E/2 + 3E^2/8)), H' = W^H H W; mixed path: one FP64 Jacobi sweep or
+//     the loose completion in its place, unless H' is diagonal to 1e-13 ||H||; FP64 path: the loose
+//     completion, H' again and the strict completion, with sweeps to the FP64 CTA Jacobi's stopping
+//     rule (np 2^-60 ||H||) where a bound fails; U = W J, ascending order and canonical phases.  The
+//     products run on the FP64 tensor cores (dmma_product).
 // GW: the working set lives in global memory (gscratch, one stride per CTA) when it does not fit
 // shared memory.
 // ---------------------------------------------------------------------------------------------

@@ -216,6 +216,8 @@ struct wnlqg_plan {
     size_t osort_bytes = 0;
     cudaStream_t stream = nullptr;
     std::vector<cudaEvent_t> events;
+    void *h_stage = nullptr;                  // pinned staging of copy_to_host (two halves), lazily allocated
+    cudaEvent_t h_stage_ev[2] = {nullptr, nullptr};
     size_t timing_batches = 0;
     int64_t launches = 0;
     bool timing_valid = false;
@@ -1339,6 +1341,9 @@ wnlqg_status wnlqg_b200_plan_destroy(wnlqg_plan *pl) {
                       (void *)pl->d_fd_tiles})
         if (ptr) cudaFree(ptr);
     for (cudaEvent_t ev : pl->events) cudaEventDestroy(ev);
+    for (cudaEvent_t ev : pl->h_stage_ev)
+        if (ev) cudaEventDestroy(ev);
+    if (pl->h_stage) cudaFreeHost(pl->h_stage);
     if (pl->stream) cudaStreamDestroy(pl->stream);
     delete pl;
     return WNLQG_OK;
@@ -2001,9 +2006,9 @@ wnlqg_status wnlqg_b200_plan_create(wnlqg_model *model, const wnlqg_task_desc *t
         return WNLQG_OK;
     };
     pl->eigh_threads = eigh_block_threads(nw);
-    // Up to 32 orbitals (orthogonal models) both precisions use the warp eigensolver: FP32 Jacobi,
-    // then FP64 refinement (one sweep on the mixed path, sweeps to FP64 convergence on the FP64
-    // path).  WNLQG_B200_CTA_EIGH=1 keeps the FP64 CTA Jacobi on the FP64 path.
+    // Up to 32 orbitals the warp eigensolvers: on the FP64 path one FP64 kernel up to 16 orbitals and
+    // the one-sided FP32 stage with the FP64 refinement above, on the mixed path the two-sided FP32
+    // stage with its refinement.  WNLQG_B200_CTA_EIGH=1 keeps the FP64 CTA Jacobi on the FP64 path.
     {
         const char *cta = std::getenv("WNLQG_B200_CTA_EIGH");
         const bool cta_fp64 = cta && cta[0] == '1' && t.precision != WNLQG_PRECISION_MIXED;
@@ -2525,8 +2530,62 @@ wnlqg_status wnlqg_b200_eval_mesh_weighted(wnlqg_plan *pl, const int64_t mesh[3]
     return WNLQG_OK;
 }
 
-wnlqg_status wnlqg_b200_eval_spectrum(wnlqg_plan *pl, const double *kpoints, int64_t n, double *energies,
-                                      double *eigenvectors) {
+}  // extern "C"
+
+namespace {
+
+// out[b][row][col] = U[b][col][row].
+__global__ void transpose_vectors_kernel(const double2 *__restrict__ U, int64_t nb, int nw, double2 *__restrict__ out) {
+    const int64_t nn = (int64_t)nw * nw, e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (e >= nb * nn) return;
+    const int64_t b = e / nn;
+    const int r = (int)(e - b * nn);
+    out[b * nn + (int64_t)(r % nw) * nw + r / nw] = U[e];
+}
+
+// Device memory to pageable host memory on the plan's stream, complete on return: in chunks through two
+// pinned halves kept by the plan, the host copying one chunk out while the next is on its way (the
+// driver's own staging of a pageable destination took 1.2 ms for 9 MB of fresh memory; 601 points of 31
+// orbitals, spectrum and vectors, 2.9 -> 1.3 ms with this and the device transposition).
+// Without pinned memory the plain copy.
+wnlqg_status copy_to_host(wnlqg_plan *pl, void *dst, const void *src, size_t bytes) {
+    constexpr size_t half = (size_t)2 << 20;
+    if (!pl->h_stage && bytes > (size_t)(64 << 10)) {
+        if (cudaMallocHost(&pl->h_stage, 2 * half) != cudaSuccess) {
+            cudaGetLastError();
+            pl->h_stage = nullptr;
+        }
+        for (int i = 0; i < 2 && pl->h_stage; ++i)
+            if (!pl->h_stage_ev[i]) WNLQG_CUDA(cudaEventCreateWithFlags(&pl->h_stage_ev[i], cudaEventDisableTiming));
+    }
+    if (!pl->h_stage || bytes <= (size_t)(64 << 10)) {
+        WNLQG_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, pl->stream));
+        WNLQG_CUDA(cudaStreamSynchronize(pl->stream));
+        return WNLQG_OK;
+    }
+    unsigned char *stage = static_cast<unsigned char *>(pl->h_stage);
+    const size_t chunks = (bytes + half - 1) / half;
+    auto issue = [&](size_t c) -> wnlqg_status {
+        const size_t off = c * half, len = std::min(half, bytes - off);
+        WNLQG_CUDA(cudaMemcpyAsync(stage + (c & 1) * half, static_cast<const unsigned char *>(src) + off, len,
+                                   cudaMemcpyDeviceToHost, pl->stream));
+        WNLQG_CUDA(cudaEventRecord(pl->h_stage_ev[c & 1], pl->stream));
+        return WNLQG_OK;
+    };
+    wnlqg_status st;
+    for (size_t c = 0; c < std::min<size_t>(2, chunks); ++c)
+        if ((st = issue(c)) != WNLQG_OK) return st;
+    for (size_t c = 0; c < chunks; ++c) {
+        const size_t off = c * half, len = std::min(half, bytes - off);
+        WNLQG_CUDA(cudaEventSynchronize(pl->h_stage_ev[c & 1]));
+        std::memcpy(static_cast<unsigned char *>(dst) + off, stage + (c & 1) * half, len);
+        if (c + 2 < chunks && (st = issue(c + 2)) != WNLQG_OK) return st;
+    }
+    return WNLQG_OK;
+}
+
+wnlqg_status eval_spectrum(wnlqg_plan *pl, const double *kpoints, int64_t n, double *energies, double *eigenvectors,
+                           bool rows) {
     wnlqg_status st = check_plan(pl);
     if (st != WNLQG_OK) return st;
     if (n < 0 || (n > 0 && (!kpoints || !energies))) return fail(WNLQG_ERR_INVALID_ARGUMENT, "invalid points");
@@ -2543,9 +2602,18 @@ wnlqg_status wnlqg_b200_eval_spectrum(wnlqg_plan *pl, const double *kpoints, int
                                        pl->stream));
         WNLQG_CUDA(cudaMemcpyAsync(energies + s * pl->nw, pl->d_E, (size_t)nb * pl->nw * sizeof(double),
                                    cudaMemcpyDeviceToHost, pl->stream));
-        if (eigenvectors)
-            WNLQG_CUDA(cudaMemcpyAsync(eigenvectors + 2 * s * pl->nn, pl->d_U, (size_t)nb * pl->nn * sizeof(double2),
-                                       cudaMemcpyDeviceToHost, pl->stream));
+        if (eigenvectors) {
+            const double2 *src = pl->d_U;
+            if (rows) {
+                // The channels are spent once the vectors exist: their buffer takes the transposes.
+                transpose_vectors_kernel<<<(unsigned)((nb * pl->nn + 255) / 256), 256, 0, pl->stream>>>(pl->d_U, nb, pl->nw,
+                                                                                                     pl->d_xw);
+                WNLQG_CUDA(cudaGetLastError());
+                src = pl->d_xw;
+            }
+            if ((st = copy_to_host(pl, eigenvectors + 2 * s * pl->nn, src, (size_t)nb * pl->nn * sizeof(double2))) != WNLQG_OK)
+                return st;
+        }
     }
     WNLQG_CUDA(cudaStreamSynchronize(pl->stream));
     pl->timing_valid = false;
@@ -2553,6 +2621,25 @@ wnlqg_status wnlqg_b200_eval_spectrum(wnlqg_plan *pl, const double *kpoints, int
     if (pl->nonorth)
         for (int v : stat)
             if (v) return fail(WNLQG_ERR_INVALID_ARGUMENT, "effective S(k) is not positive definite");
+    return WNLQG_OK;
+}
+
+}  // namespace
+
+extern "C" {
+
+wnlqg_status wnlqg_b200_eval_spectrum_rows(wnlqg_plan *pl, const double *kpoints, int64_t n, double *energies,
+                                           double *eigenvectors) {
+    wnlqg_status st = check_plan(pl);
+    if (st != WNLQG_OK) return st;
+    if (pl->conv1) return fail(WNLQG_ERR_UNSUPPORTED, "row-major vectors in Convention I are not built");
+    return eval_spectrum(pl, kpoints, n, energies, eigenvectors, true);
+}
+
+wnlqg_status wnlqg_b200_eval_spectrum(wnlqg_plan *pl, const double *kpoints, int64_t n, double *energies,
+                                      double *eigenvectors) {
+    wnlqg_status st = eval_spectrum(pl, kpoints, n, energies, eigenvectors, false);
+    if (st != WNLQG_OK) return st;
     if (pl->conv1 && eigenvectors) {
         // Convention I eigenvectors: D(k)^H U, D = diag(exp(2 pi i k.tau_frac)) (the similarity of
         // _apply_wannier_center_similarity!), then the canonical phase rule again

@@ -139,11 +139,16 @@ class ResponseEngine:
         k = np.ascontiguousarray(np.asarray(kpoints, dtype=np.float64).reshape(-1, 3))
         nw = self.model.num_orbitals
         e = np.zeros((k.shape[0], nw))
-        # Column-major per k: store as [n, col, row] and transpose.
-        u = np.zeros((k.shape[0], nw, nw), dtype=np.complex128) if vectors else None
         dp = ctypes.POINTER(ctypes.c_double)
-        _lib.check(self._L.wnlqg_b200_eval_spectrum(self._plan, k.ctypes.data_as(dp), k.shape[0], e.ctypes.data_as(dp),
-                                                    u.ctypes.data_as(dp) if vectors else None))
+        kp, ep = k.ctypes.data_as(dp), e.ctypes.data_as(dp)
+        if vectors and self.task.desc.wannier_center_convention == 0:
+            # Row-major vectors: the device transposes them, the host writes the array once.
+            u = np.empty((k.shape[0], nw, nw), dtype=np.complex128)
+            _lib.check(self._L.wnlqg_b200_eval_spectrum_rows(self._plan, kp, k.shape[0], ep, u.ctypes.data_as(dp)))
+            return e, u
+        # Column-major per k: stored as [n, col, row] and transposed.
+        u = np.zeros((k.shape[0], nw, nw), dtype=np.complex128) if vectors else None
+        _lib.check(self._L.wnlqg_b200_eval_spectrum(self._plan, kp, k.shape[0], ep, u.ctypes.data_as(dp) if vectors else None))
         return e, (np.ascontiguousarray(u.transpose(0, 2, 1)) if vectors else None)
 
     def last_timing(self):
