@@ -9,7 +9,12 @@
 // start from a neighbouring point's V takes one product instead of four.
 //   - H is scaled by a power of two to a Frobenius norm in [1/2, 1), so no square leaves the FP32 range.
 //   - A sweep is the last when no pair above the rounding level (cosine 2^-20) turned by more than
-//     OS_ANGLE: convergence is quadratic, so it leaves angles of about the square of that.
+//     an angle: convergence is quadratic, but what the last sweep leaves adds up over the columns.
+//     With every pair just below 2^-10, as between neighbours of a dense mesh, ||V^H V - 1|| came to
+//     3e-5 (32 orbitals) and 9e-5 (128), of which the FP64 stage's second-order orthonormalisation
+//     leaves 1e-14 and 1e-13, and ratios a_ij / (d_i - d_j) to 3e-4 and 1e-3, which its first completion
+//     refuses.  2^-11 up to 32 orbitals and 2^-12 above leave at most 8e-6 (3e-16 after the FP64 stage)
+//     and ratios below 1e-4.
 //   - The angle left by rounding is about 2^-24 (lambda + c) / (difference of two levels), so a tighter
 //     c is a more accurate start.  A cold start takes c = 1.1 ||H||_F, a warm one 1.3 max |lambda| of
 //     the columns it starts from; above 32 orbitals a converged cold start is followed by a warm one
@@ -17,9 +22,8 @@
 //   - The start V has to be orthonormal (G G^H = (H + c I)^2): it always is a converged one.
 //   - Should a column shrink below 0.05 c (H moved beyond the shift along a chain), the point is
 //     restarted with the shift of its own columns.
-// Emulated in numpy FP32 on the workload's matrices (32, 64 and 96 orbitals): 2 to 4 sweeps warm, 6 to 8
-// cold, vectors orthonormal to 5e-7 and off-diagonal elements of V^H H V within 1e-5 (32) to 1e-4 (96)
-// of the level differences, below the 2^-13 that the FP64 stage's first completion asks for.
+// On random spectra the vectors are otherwise orthonormal to 4e-7 (18 orbitals) to 1.2e-6 (128), ratios
+// 3e-6 to 7e-5: below the 2^-13 that the FP64 stage's first completion asks for.
 // Measured against the two-sided stage: 32 orbitals, 32768 points of a 256^3 mesh, 6.9 -> 2.5 ms; 96
 // orbitals, 2048 points, 44.4 -> 5.8 ms (and the FP64 stage, which no longer needs a sweep before its
 // completion, 32.5 -> 10.2 ms).
@@ -27,14 +31,15 @@
 #include "common.cuh"
 #include "regjacobi.cuh"
 
-#define OS_ANGLE 0.0009765625f      // 2^-10
+#define OS_ANGLE_WARP 4.8828125e-04f      // 2^-11
+#define OS_ANGLE_CTA 2.44140625e-04f      // 2^-12
 #define OS_MAX_SWEEPS 20
 #define OS_RESTARTS 3
 
 // The rotation of a pair with Gram matrix [nx, a; conj(a), ny]; a at or below the rounding level of the
-// two norms is left (c = 1, s = 0).  Returns whether the pair turned by more than OS_ANGLE; shift =
+// two norms is left (c = 1, s = 0).  Returns whether the pair turned by more than `angle`; shift =
 // t |a| is what ny gains and nx loses.
-WNLQG_D bool os_rotation(float2 a, float nx, float ny, float &c, float2 &s, float &shift) {
+WNLQG_D bool os_rotation(float2 a, float nx, float ny, float angle, float &c, float2 &s, float &shift) {
     const float a2 = a.x * a.x + a.y * a.y;
     c = 1.0f;
     s = make_float2(0.0f, 0.0f);
@@ -47,7 +52,7 @@ WNLQG_D bool os_rotation(float2 a, float nx, float ny, float &c, float2 &s, floa
     const float sg = t * c * inv;
     s = make_float2(sg * a.x, sg * a.y);
     shift = t * (a2 * inv);
-    return a2 > 9.0949470e-13f * (nx * ny) && fabsf(t) > OS_ANGLE;    // cosine 2^-20
+    return a2 > 9.0949470e-13f * (nx * ny) && fabsf(t) > angle;    // cosine 2^-20
 }
 
 WNLQG_D void os_rotate(float2 &x, float2 &y, float c, float2 s) {
@@ -107,7 +112,7 @@ template <int NP> WNLQG_D float os_norms(const float2 (&g)[NP]) {
     return (threadIdx.x & 1) ? n.y : n.x;
 }
 
-// One sweep; returns whether a pair turned by more than OS_ANGLE.
+// One sweep; returns whether a pair turned by more than OS_ANGLE_WARP.
 template <int NP> WNLQG_D bool os_sweep(float2 (&g)[NP], float4 (*rot)[16]) {
     constexpr int H = NP / 2;
     const int lane = threadIdx.x & 31, m = lane >> 1;
@@ -136,7 +141,7 @@ template <int NP> WNLQG_D bool os_sweep(float2 (&g)[NP], float4 (*rot)[16]) {
         const float other = __shfl_xor_sync(0xffffffffu, n, 1);
         float c, shift;
         float2 s;
-        const bool turned = os_rotation(a, (lane & 1) ? other : n, (lane & 1) ? n : other, c, s, shift);
+        const bool turned = os_rotation(a, (lane & 1) ? other : n, (lane & 1) ? n : other, OS_ANGLE_WARP, c, s, shift);
         big = big || turned;
         n += (lane & 1) ? shift : -shift;
         float4 *r = rot[round & 1];
@@ -332,7 +337,7 @@ WNLQG_D bool os_round4(float2 (&g)[8][RP], float (&n)[8]) {
     const float ny = q < 2 ? (q == 0 ? n[Y0] : n[Y1]) : (q == 2 ? n[Y2] : n[Y3]);
     float c, shift;
     float2 s;
-    const bool turned = os_rotation(a, nx, ny, c, s, shift);
+    const bool turned = os_rotation(a, nx, ny, OS_ANGLE_CTA, c, s, shift);
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
         const float ck = __shfl_sync(0xffffffffu, c, 8 * k), hk = __shfl_sync(0xffffffffu, shift, 8 * k);
@@ -377,7 +382,7 @@ __global__ void __launch_bounds__(RP == 2 ? 256 : (RP == 3 ? 384 : 512), RP == 2
 #pragma unroll
             for (int r = 0; r < RP; ++r) G[(size_t)((q < 4 ? cI + q : cJ + q - 4)) * LR + lane + 32 * r] = g[q][r];
     };
-    // One sweep; returns (in every thread) whether a pair turned by more than OS_ANGLE.
+    // One sweep; returns (in every thread) whether a pair turned by more than OS_ANGLE_CTA.
     auto sweep = [&]() -> bool {
         bool big = false;
 #pragma unroll 1
