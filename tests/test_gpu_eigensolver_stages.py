@@ -43,6 +43,33 @@ def check_spectrum(h, e, u):
     assert np.max(np.abs(u.conj().T @ u - np.eye(len(e)))) <= 1e-13
 
 
+def skewed(rng, nw, scales):
+    """One deep level and a band of others, slowly rotating, with the given scales."""
+    q, h = unitary(rng, nw), []
+    for s in scales:
+        h.append(s * (q * np.r_[-1.0, np.linspace(-0.25, 0.25, nw - 1)]) @ q.conj().T)
+        q = unitary(rng, nw, 1e-3) @ q
+    return np.array([0.5 * (x + x.conj().T) for x in h])
+
+
+@pytest.mark.parametrize("chain", ["falling", "rising", "jumps"])
+@pytest.mark.parametrize("nw", [20, 31, 40, 96])
+def test_warm_chain_whose_norm_moves(stages, nw, chain):
+    rng = np.random.default_rng(nw)
+    if chain == "jumps":
+        scales = [1.0, 5.0, 0.1, -1.0, 1.0, 0.0, 2.0, -0.3, -8.0, 1e-20, 1.0, -1e20, 3.0, 0.0, 0.0, 1e-3]
+    else:
+        scales = 1.5 * 0.98 ** np.arange(150)
+        scales = scales if chain == "falling" else scales[::-1]
+    h = skewed(rng, nw, scales)
+    v, e, u = native.run(stages, h)
+    got = np.array([stage1_quality(a, b) for a, b, s in zip(h, v, scales) if s != 0.0])
+    assert np.max(got[:, 0]) <= ORTHONORMAL
+    assert np.max(got[:, 1]) <= RATIO
+    for i in range(0, len(h), 1 if chain == "jumps" else 7):
+        check_spectrum(h[i], e[i], u[i])
+
+
 @pytest.mark.parametrize("nw", [18, 32, 64, 96, 128])
 @pytest.mark.parametrize("angle", [1e-2, 9e-4, 4.7e-4, 2.3e-4])
 def test_warm_start_from_close_neighbours(stages, nw, angle):

@@ -17,15 +17,17 @@
 //     and ratios below 1e-4.
 //   - The angle left by rounding is about 2^-24 (lambda + c) / (difference of two levels), so a tighter
 //     c is a more accurate start.  A cold start takes c = 1.1 ||H||_F, a warm one 1.3 max |lambda| of
-//     the columns it starts from; above 32 orbitals a converged cold start is followed by a warm one
-//     from its own vectors.
+//     the columns it starts from (in the present point's scaling); above 32 orbitals a start with a
+//     loose c (a cold one, or max |lambda| fell along the chain) is followed by one from its own vectors.
 //   - The start V has to be orthonormal (G G^H = (H + c I)^2): it always is a converged one.
-//   - Should a column shrink below 0.05 c (H moved beyond the shift along a chain), the point is
-//     restarted with the shift of its own columns.
+//   - H + c I has to be definite: of an indefinite one the lengths are |lambda + c|, and two levels of
+//     equal length mix.  H may have moved beyond the shift along a chain, so a warm point is accepted
+//     only if no column is shorter than 0.05 c and the lengths sum to tr(H + c I) within 0.05 c (a
+//     level below -c would add twice its length); else it is started cold.
 // On random spectra the vectors are otherwise orthonormal to 4e-7 (18 orbitals) to 1.2e-6 (128), ratios
 // 3e-6 to 7e-5: below the 2^-13 that the FP64 stage's first completion asks for.
 // Measured against the two-sided stage: 32 orbitals, 32768 points of a 256^3 mesh, 6.9 -> 2.5 ms; 96
-// orbitals, 2048 points, 44.4 -> 5.8 ms (and the FP64 stage, which no longer needs a sweep before its
+// orbitals, 2048 points, 44.4 -> 6.1 ms (and the FP64 stage, which no longer needs a sweep before its
 // completion, 32.5 -> 10.2 ms).
 #pragma once
 #include "common.cuh"
@@ -34,7 +36,6 @@
 #define OS_ANGLE_WARP 4.8828125e-04f      // 2^-11
 #define OS_ANGLE_CTA 2.44140625e-04f      // 2^-12
 #define OS_MAX_SWEEPS 20
-#define OS_RESTARTS 3
 
 // The rotation of a pair with Gram matrix [nx, a; conj(a), ny]; a at or below the rounding level of the
 // two norms is left (c = 1, s = 0).  Returns whether the pair turned by more than `angle`; shift =
@@ -70,6 +71,16 @@ WNLQG_D float os_scale(double fro) {
     frexp(fro, &e);
     e = max(-120, min(120, e));
     return ldexpf(1.0f, -e);
+}
+
+// The shift of a point that starts cold, and of one that starts from vectors with max |lambda| = lmax in
+// the present scaling.
+WNLQG_D float os_cold_shift(double fro, float sc) { return 1.1f * (float)fmax(fro * (double)sc, 0.5); }
+WNLQG_D float os_warm_shift(float lmax) { return fmaxf(1.3f * lmax, 0.01f); }
+
+// Whether H + c I is definite, from the smallest and the sum of its columns' lengths and its trace.
+WNLQG_D bool os_definite(float smallest, float sum, float trace, float shift) {
+    return smallest >= 0.05f * shift && fabsf(sum - trace) <= 0.05f * shift;
 }
 
 // Sum over the warp of the complex v[0 .. 15], scattered: lanes 2m and 2m + 1 get v[m].
@@ -177,20 +188,21 @@ __global__ void __launch_bounds__(128, 3) onesided_warp_kernel(const double2 *__
     if (w >= chains) return;   // whole warps
     const int64_t kb = (batch * w) / chains, ke = (batch * (w + 1)) / chains;
     float2 g[NP];
-    float shift = 0.0f;
-    // g <- its normalised columns (a zero column, which only a zero H has, becomes the unit vector),
-    // their largest |lambda| and smallest length.
-    auto normalise = [&](float &lmax, float &smin) {
+    float shift = 0.0f, lmax = 0.0f, sc_before = 1.0f;
+    // g <- its normalised columns, lmax their largest |lambda|; returns whether H + c I is definite
+    // (h_trace: tr H).
+    auto normalise = [&](float h_trace) -> bool {
         const float n2 = os_norms<NP>(g);
         const int m = i >> 1;
         const bool held = m < NP / 2;
         const float len = sqrtf(n2);
+        float smin = held ? len : 3.0e38f, sum = held ? len : 0.0f;
         lmax = held ? fabsf(len - shift) : 0.0f;
-        smin = held ? len : 3.0e38f;
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) {
             lmax = fmaxf(lmax, __shfl_xor_sync(0xffffffffu, lmax, o));
             smin = fminf(smin, __shfl_xor_sync(0xffffffffu, smin, o));
+            sum += __shfl_xor_sync(0xffffffffu, sum, o);
         }
         __syncwarp();
         if (held) sm.inv[(i & 1) ? NP - 1 - m : m] = n2 > 0.0f ? rsqrtf(n2) : 0.0f;
@@ -198,63 +210,66 @@ __global__ void __launch_bounds__(128, 3) onesided_warp_kernel(const double2 *__
 #pragma unroll
         for (int j = 0; j < NP; ++j) {
             const float f = sm.inv[j];
-            g[j] = f > 0.0f ? make_float2(g[j].x * f, g[j].y * f) : make_float2(j == i ? 1.0f : 0.0f, 0.0f);
+            g[j] = make_float2(g[j].x * f, g[j].y * f);
         }
+        return __all_sync(0xffffffffu, os_definite(smin, sum, h_trace + NP * shift, shift));
     };
-    float lmax = 0.0f, smin = 0.0f;
     for (int64_t b = kb; b < ke; ++b) {
         __syncwarp();
         reg_stage_hermitian<float, NP>(sm.S2, h_in + b * h_stride, nw, true);
-        double f2 = 0.0;
+        double f2 = 0.0, trace = 0.0;
         for (int j = 0; j < NP; ++j) {
             const float2 z = sm.S2[j * LD + ic];
             f2 += (double)z.x * z.x + (double)z.y * z.y;
+            if (j == i) trace = z.x;
         }
         if (i >= NP) f2 = 0.0;
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) f2 += __shfl_xor_sync(0xffffffffu, f2, o);
+        for (int o = 16; o > 0; o >>= 1) {
+            f2 += __shfl_xor_sync(0xffffffffu, f2, o);
+            trace += __shfl_xor_sync(0xffffffffu, trace, o);
+        }
         const double fro = sqrt(f2);
-        const float sc = os_scale(fro), cold_shift = 1.1f * (float)fmax(fro * (double)sc, 0.5);
-        if (b == kb || !warm_start) {
-            shift = cold_shift;
+        const float sc = os_scale(fro), cold_shift = os_cold_shift(fro, sc);
+        bool cold = b == kb || !warm_start;
+        for (;;) {
+            if (cold) {
+                shift = cold_shift;
 #pragma unroll
-            for (int j = 0; j < NP; ++j) {
-                const float2 z = sm.S2[j * LD + ic];   // H[i][j] = conj(H[j][i])
-                g[j] = make_float2(sc * z.x + (j == i ? shift : 0.0f), -sc * z.y);
-                if (i >= NP) g[j] = make_float2(0.0f, 0.0f);
-            }
-            for (int sweep = 0; sweep < OS_MAX_SWEEPS; ++sweep)
-                if (!os_sweep<NP>(g, sm.rot)) break;
-            normalise(lmax, smin);
-        }
-        const bool cold = b == kb || !warm_start;
-        for (int restart = cold ? OS_RESTARTS : 0; restart < OS_RESTARTS; ++restart) {
-            // g <- (H + c I) V.
-            shift = fmaxf(1.3f * lmax, 0.01f);
-            if (i < NP)
-#pragma unroll
-                for (int j = 0; j < NP; j += 2)
-                    *reinterpret_cast<float4 *>(sm.S1 + i * LD + j) = make_float4(g[j].x, g[j].y, g[j + 1].x, g[j + 1].y);
-            __syncwarp();
-#pragma unroll
-            for (int j = 0; j < NP; ++j) g[j] = make_float2(shift * g[j].x, shift * g[j].y);
-#pragma unroll 1
-            for (int l = 0; l < NP; ++l) {
-                const float2 z = sm.S2[l * LD + ic];
-                const float2 h = i < NP ? make_float2(sc * z.x, -sc * z.y) : make_float2(0.0f, 0.0f);
-#pragma unroll
-                for (int j = 0; j < NP; j += 2) {
-                    const float4 y = *reinterpret_cast<const float4 *>(sm.S1 + l * LD + j);
-                    g[j] = cfma(h, make_float2(y.x, y.y), g[j]);
-                    g[j + 1] = cfma(h, make_float2(y.z, y.w), g[j + 1]);
+                for (int j = 0; j < NP; ++j) {
+                    const float2 z = sm.S2[j * LD + ic];   // H[i][j] = conj(H[j][i])
+                    g[j] = make_float2(sc * z.x + (j == i ? shift : 0.0f), -sc * z.y);
+                    if (i >= NP) g[j] = make_float2(0.0f, 0.0f);
                 }
+            } else {
+                // g <- (H + c I) V.
+                shift = fminf(os_warm_shift(lmax * (sc / sc_before)), cold_shift);
+                if (i < NP)
+#pragma unroll
+                    for (int j = 0; j < NP; j += 2)
+                        *reinterpret_cast<float4 *>(sm.S1 + i * LD + j) = make_float4(g[j].x, g[j].y, g[j + 1].x, g[j + 1].y);
+                __syncwarp();
+#pragma unroll
+                for (int j = 0; j < NP; ++j) g[j] = make_float2(shift * g[j].x, shift * g[j].y);
+#pragma unroll 1
+                for (int l = 0; l < NP; ++l) {
+                    const float2 z = sm.S2[l * LD + ic];
+                    const float2 h = i < NP ? make_float2(sc * z.x, -sc * z.y) : make_float2(0.0f, 0.0f);
+#pragma unroll
+                    for (int j = 0; j < NP; j += 2) {
+                        const float4 y = *reinterpret_cast<const float4 *>(sm.S1 + l * LD + j);
+                        g[j] = cfma(h, make_float2(y.x, y.y), g[j]);
+                        g[j + 1] = cfma(h, make_float2(y.z, y.w), g[j + 1]);
+                    }
+                }
+                __syncwarp();
             }
-            __syncwarp();
             for (int sweep = 0; sweep < OS_MAX_SWEEPS; ++sweep)
                 if (!os_sweep<NP>(g, sm.rot)) break;
-            normalise(lmax, smin);
-            if (!(smin < 0.05f * shift)) break;
+            if (normalise((float)(trace * (double)sc)) || cold) break;
+            cold = true;
         }
+        sc_before = sc;
         if (i < NP) {
             float2 *vo = V_out + b * (int64_t)NP * NP;
 #pragma unroll
@@ -358,7 +373,7 @@ __global__ void __launch_bounds__(RP == 2 ? 256 : (RP == 3 ? 384 : 512), RP == 2
     onesided_cta_kernel(const double2 *__restrict__ h_in, int64_t h_stride, int64_t batch, int nw,
                         float2 *__restrict__ V_out, int warm_start) {
     extern __shared__ __align__(16) unsigned char os_smem_raw[];
-    __shared__ float red[2][16];
+    __shared__ float red[3][16];
     __shared__ double dred[16];
     constexpr int LR = OS_ROWS(RP);
     const int np = nw + (nw & 1);
@@ -367,7 +382,7 @@ __global__ void __launch_bounds__(RP == 2 ? 256 : (RP == 3 ? 384 : 512), RP == 2
     float2 *Hp = G + (size_t)ncol * LR;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
     const int64_t kb = (batch * (int64_t)blockIdx.x) / gridDim.x, ke = (batch * ((int64_t)blockIdx.x + 1)) / gridDim.x;
-    float shift = 0.0f, lmax = 0.0f, smin = 0.0f;
+    float shift = 0.0f, lmax = 0.0f, sc_before = 1.0f;
     float2 g[8][RP];
     float n[8];
     auto load8 = [&](int cI, int cJ) {
@@ -409,36 +424,41 @@ __global__ void __launch_bounds__(RP == 2 ? 256 : (RP == 3 ? 384 : 512), RP == 2
         }
         return __syncthreads_or(big ? 1 : 0) != 0;
     };
-    // Columns normalised in place (a zero column j < np, which only a zero H has, becomes the unit
-    // vector); largest |lambda| and smallest length over the np columns, in every thread.
-    auto normalise = [&]() {
-        float lm = 0.0f, sn = 3.0e38f;
+    // Columns normalised in place, lmax their largest |lambda|; returns whether H + c I is definite
+    // (h_trace: tr H), all over the np columns and in every thread.
+    auto normalise = [&](float h_trace) -> bool {
+        float lm = 0.0f, smin = 3.0e38f, sum = 0.0f;
         for (int k = warp; k < nblk / 2; k += nwarps) {
             load8(8 * k, 8 * k + 4);
             os_norms8<RP>(g, n);
 #pragma unroll
             for (int q = 0; q < 8; ++q) {
-                const int j = 8 * k + q;
-                if (j < np) {
+                if (8 * k + q < np) {
                     const float len = sqrtf(n[q]);
                     lm = fmaxf(lm, fabsf(len - shift));
-                    sn = fminf(sn, len);
+                    smin = fminf(smin, len);
+                    sum += len;
                 }
                 const float f = n[q] > 0.0f ? rsqrtf(n[q]) : 0.0f;
 #pragma unroll
-                for (int r = 0; r < RP; ++r)
-                    g[q][r] = f > 0.0f ? make_float2(g[q][r].x * f, g[q][r].y * f)
-                                       : make_float2(j < np && lane + 32 * r == j ? 1.0f : 0.0f, 0.0f);
+                for (int r = 0; r < RP; ++r) g[q][r] = make_float2(g[q][r].x * f, g[q][r].y * f);
             }
             store8(8 * k, 8 * k + 4);
         }
-        if (lane == 0) { red[0][warp] = lm; red[1][warp] = sn; }
+        if (lane == 0) { red[0][warp] = lm; red[1][warp] = smin; red[2][warp] = sum; }
         __syncthreads();
         lmax = 0.0f;
         smin = 3.0e38f;
-        for (int w = 0; w < nwarps; ++w) { lmax = fmaxf(lmax, red[0][w]); smin = fminf(smin, red[1][w]); }
+        sum = 0.0f;
+        for (int w = 0; w < nwarps; ++w) {
+            lmax = fmaxf(lmax, red[0][w]);
+            smin = fminf(smin, red[1][w]);
+            sum += red[2][w];
+        }
         __syncthreads();
+        return os_definite(smin, sum, h_trace + np * shift, shift);
     };
+    bool redo = false;
     for (int64_t b = kb; b < ke; ++b) {
         const double2 *h = h_in + b * h_stride;
         double f2 = 0.0;
@@ -457,14 +477,22 @@ __global__ void __launch_bounds__(RP == 2 ? 256 : (RP == 3 ? 384 : 512), RP == 2
         double fro = 0.0;
         for (int w = 0; w < nwarps; ++w) fro += dred[w];
         fro = sqrt(fro);
-        const float sc = os_scale(fro);
+        const float sc = os_scale(fro), cold_shift = os_cold_shift(fro, sc);
+        float h_trace = 0.0f;
+        for (int j = lane; j < np; j += 32) h_trace += sc * Hp[(size_t)j * (j + 1) / 2 + j].x;
+        for (int o = 16; o > 0; o >>= 1) h_trace += __shfl_xor_sync(0xffffffffu, h_trace, o);
         auto h_elem = [&](int r, int l) -> float2 {   // scaled H[r][l]
             if (r >= np) return make_float2(0.0f, 0.0f);
             const float2 z = r <= l ? Hp[(size_t)l * (l + 1) / 2 + r] : Hp[(size_t)r * (r + 1) / 2 + l];
             return make_float2(sc * z.x, r <= l ? sc * z.y : -sc * z.y);
         };
-        if (b == kb || !warm_start) {
-            shift = 1.1f * (float)fmax(fro * (double)sc, 0.5);
+        lmax *= sc / sc_before;
+        sc_before = sc;
+        // Also cold where max |lambda| fell so far that the warm shift would be the looser one.
+        const bool cold = b == kb || !warm_start || redo || !(lmax <= cold_shift);
+        redo = false;
+        if (cold) {
+            shift = cold_shift;
             for (int e = threadIdx.x; e < ncol * LR; e += blockDim.x) {
                 const int j = e / LR, r = e % LR;
                 float2 z = make_float2(0.0f, 0.0f);
@@ -477,11 +505,12 @@ __global__ void __launch_bounds__(RP == 2 ? 256 : (RP == 3 ? 384 : 512), RP == 2
             __syncthreads();
             for (int s = 0; s < OS_MAX_SWEEPS; ++s)
                 if (!sweep()) break;
-            normalise();
+            normalise(h_trace);
         }
-        for (int restart = 0; restart < OS_RESTARTS; ++restart) {
+        bool definite = true;
+        for (int start = 0; start < 2; ++start) {
             // G <- (H + c I) V: a warp needs its own eight columns of V only.
-            shift = fmaxf(1.3f * lmax, 0.01f);
+            shift = os_warm_shift(lmax);
             for (int k = warp; k < nblk / 2; k += nwarps) {
                 load8(8 * k, 8 * k + 4);
 #pragma unroll
@@ -507,8 +536,13 @@ __global__ void __launch_bounds__(RP == 2 ? 256 : (RP == 3 ? 384 : 512), RP == 2
             __syncthreads();
             for (int s = 0; s < OS_MAX_SWEEPS; ++s)
                 if (!sweep()) break;
-            normalise();
-            if (!(smin < 0.05f * shift)) break;
+            definite = normalise(h_trace);
+            if (!definite || shift <= 1.5f * lmax) break;
+        }
+        if (!definite && !cold) {   // again from a cold start
+            redo = true;
+            --b;
+            continue;
         }
         float2 *vo = V_out + b * (int64_t)np * np;
         for (int j = warp; j < np; j += nwarps)
