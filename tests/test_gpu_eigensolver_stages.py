@@ -1,5 +1,5 @@
 """The FP64 path's two eigensolver stages on chosen matrices (17 orbitals and more): what stage 1 leaves
-along a chain of warm starts, and the spectra that stage 2 makes of it."""
+along a chain of warm starts, and the spectra that stage 2 makes of it and of starts at its bounds."""
 import numpy as np
 import pytest
 
@@ -85,3 +85,21 @@ def test_warm_start_from_close_neighbours(stages, nw, angle):
     assert np.max(got[:, 0]) <= ORTHONORMAL
     assert np.max(got[:, 1]) <= RATIO
     check_spectrum(h[-1], e[-1], u[-1])
+
+
+@pytest.mark.parametrize("nw", [17, 32, 64, 96, 128])
+@pytest.mark.parametrize("ratio", [1e-6, 1e-5, 3e-5, 7e-5])
+@pytest.mark.parametrize("coherent", [True, False])
+def test_every_pair_near_the_completion_bound(stages, nw, ratio, coherent):
+    """Starts exp(i K) away from the eigenvectors with every |K_ij| = ratio (below 2^-13): the norm of K
+    is up to nw times larger."""
+    rng = np.random.default_rng(nw)
+    q = unitary(rng, nw)
+    phase = np.zeros((nw, nw)) if coherent else rng.uniform(0.0, 2.0 * np.pi, (nw, nw))
+    k = np.triu(np.exp(1j * phase), 1)
+    w, p = np.linalg.eigh(ratio * (k + k.conj().T))
+    h = (q * np.linspace(-1.0, 1.0, nw)) @ q.conj().T
+    h = 0.5 * (h + h.conj().T)
+    start = q @ (p * np.exp(1j * w)) @ p.conj().T
+    _, e, u = native.run(stages, h[None], start=start[None])
+    check_spectrum(h, e[0], u[0])

@@ -630,8 +630,17 @@ __global__ void __launch_bounds__(TEAM == 32 ? 128 : TEAM, TEAM == 32 ? 4 : (TEA
 // whose deviation from unitarity is |E|^4 / 4 instead of |E|^2.  Returns false, with A and W
 // untouched, when some pair is too close for the bound (the caller then sweeps).  dnew: np
 // doubles of the team's scratch.
+// tau bounds the elements, and the norm of E may be np times larger: 128 levels with every ratio just
+// below 2^-13 lost 2e-9 of the vectors' orthonormality, below 2^-26 up to 4e-12.  On the FP64 path
+// (red != nullptr) norm2 therefore gets ||E||_F^2; the strict completion takes the E^2 / 2 term too
+// above COMPLETION_STRICT2, and after a loose one above COMPLETION_LOOSE2 the caller orthonormalises W
+// again.  Either keeps the deviation below 2^-46 = 1.4e-14 at any order; ratios as stage 1 leaves them
+// (||E||_F of 1e-4, then 1e-8) take neither.
+#define COMPLETION_LOOSE2 2.384185791015625e-07      // 2^-22: |E|^4 / 4 <= 2^-46
+#define COMPLETION_STRICT2 1.4210854715202004e-14    // 2^-46
 template <int TEAM>
-WNLQG_D bool team_first_order_completion(double2 *A, double2 *W, int np, int ld, double *dnew, double tau) {
+WNLQG_D bool team_first_order_completion(double2 *A, double2 *W, int np, int ld, double *dnew, double tau, double *red,
+                                         double &norm2) {
     const int t = Team<TEAM>::rank();
     bool bad = false;
     for (int e = t; e < np * np; e += TEAM) {
@@ -653,18 +662,26 @@ WNLQG_D bool team_first_order_completion(double2 *A, double2 *W, int np, int ld,
     }
     Team<TEAM>::sync();
     // A <- I + E: the off-diagonal in place (reading only the unchanged diagonal), then the diagonal.
+    double local = 0.0;
     for (int e = t; e < np * np; e += TEAM) {
         const int i = e % np, j = e / np;
         const double2 a = A[i + ld * j];
         if (i == j || (a.x == 0.0 && a.y == 0.0)) continue;
         const double g = A[j + ld * j].x - A[i + ld * i].x;
-        A[i + ld * j] = make_double2(a.x / g, a.y / g);
+        const double2 ej = make_double2(a.x / g, a.y / g);
+        local += ej.x * ej.x + ej.y * ej.y;
+        A[i + ld * j] = ej;
+    }
+    bool second = tau > 1.4901161193847656e-08;
+    if (red) {
+        norm2 = Team<TEAM>::sum(local, red);
+        second = second || norm2 > COMPLETION_STRICT2;
     }
     Team<TEAM>::sync();
     if (t < np) A[t + ld * t] = make_double2(1.0, 0.0);
     Team<TEAM>::sync();
     if constexpr (TEAM == 128) {
-        if (tau > 1.4901161193847656e-08) {
+        if (second) {
             team128_dmma<false>(A, A, A, np, ld, [](int r, int c, double2 v) {   // A <- I + E + E^2 / 2
                 return make_double2(0.5 * (v.x + (r == c ? 1.0 : 0.0)), 0.5 * v.y);
             });
@@ -676,7 +693,7 @@ WNLQG_D bool team_first_order_completion(double2 *A, double2 *W, int np, int ld,
         return true;
     }
     double2 col[Team<TEAM>::ROWS];
-    if (tau > 1.4901161193847656e-08) {
+    if (second) {
         constexpr int ROWS = Team<TEAM>::ROWS;
         const int c0 = t & 31, r0 = (t >> 5) * ROWS;
         team_column_product<TEAM>(A, A, col, np, ld, false);                // ((I + E)^2)[:, c0]
@@ -747,40 +764,43 @@ __global__ void __launch_bounds__(TEAM == 128 ? 128 : 64, TEAM == 32 ? 1 : (TEAM
             W[i + ld * j] = to_c64(vi[i + np * j]);
         }
         Team<TEAM>::sync();
-        // E = V^H V - I into A; then M = I - E/2 + 3 E^2 / 8 into A; W <- V M.
-        if constexpr (TEAM == 128) {
-            team128_dmma<true>(W, W, A, np, ld, [](int r, int c, double2 v) {
-                return make_double2(v.x - (r == c ? 1.0 : 0.0), v.y);
-            });
-            Team<TEAM>::sync();
-            team128_dmma<false>(A, A, A, np, ld, [&](int r, int c, double2 v) {      // (E^2), then M
-                const double2 e = A[r + ld * c];
-                return make_double2((r == c ? 1.0 : 0.0) - 0.5 * e.x + 0.375 * v.x, -0.5 * e.y + 0.375 * v.y);
-            });
-            Team<TEAM>::sync();
-            team128_dmma<false>(W, A, W, np, ld, [](int, int, double2 v) { return v; });   // W <- V M
-        } else {
-        team_column_product<TEAM>(W, W, col, np, ld, true);
+        // E = W^H W - I into A; then M = I - E/2 + 3 E^2 / 8 into A; W <- W M.
+        auto orthonormalise = [&]() {
+            if constexpr (TEAM == 128) {
+                team128_dmma<true>(W, W, A, np, ld, [](int r, int c, double2 v) {
+                    return make_double2(v.x - (r == c ? 1.0 : 0.0), v.y);
+                });
+                Team<TEAM>::sync();
+                team128_dmma<false>(A, A, A, np, ld, [&](int r, int c, double2 v) {      // (E^2), then M
+                    const double2 e = A[r + ld * c];
+                    return make_double2((r == c ? 1.0 : 0.0) - 0.5 * e.x + 0.375 * v.x, -0.5 * e.y + 0.375 * v.y);
+                });
+                Team<TEAM>::sync();
+                team128_dmma<false>(W, A, W, np, ld, [](int, int, double2 v) { return v; });   // W <- V M
+            } else {
+            team_column_product<TEAM>(W, W, col, np, ld, true);
 #pragma unroll
-        for (int i = 0; i < ROWS; ++i)
-            if (r0 + i == c0) col[i].x -= 1.0;
-        team_store_column<TEAM>(A, col, np, ld);
-        Team<TEAM>::sync();
-        team_column_product<TEAM>(A, A, col, np, ld, false);                 // (E^2)[:, c0]
+            for (int i = 0; i < ROWS; ++i)
+                if (r0 + i == c0) col[i].x -= 1.0;
+            team_store_column<TEAM>(A, col, np, ld);
+            Team<TEAM>::sync();
+            team_column_product<TEAM>(A, A, col, np, ld, false);                 // (E^2)[:, c0]
 #pragma unroll
-        for (int i = 0; i < ROWS; ++i) {
-            if (r0 + i < np && c0 < np) {
-                const double2 e = A[(r0 + i) + ld * c0];
-                col[i] = make_double2((r0 + i == c0 ? 1.0 : 0.0) - 0.5 * e.x + 0.375 * col[i].x, -0.5 * e.y + 0.375 * col[i].y);
+            for (int i = 0; i < ROWS; ++i) {
+                if (r0 + i < np && c0 < np) {
+                    const double2 e = A[(r0 + i) + ld * c0];
+                    col[i] = make_double2((r0 + i == c0 ? 1.0 : 0.0) - 0.5 * e.x + 0.375 * col[i].x, -0.5 * e.y + 0.375 * col[i].y);
+                }
             }
-        }
-        Team<TEAM>::sync();
-        team_store_column<TEAM>(A, col, np, ld);
-        Team<TEAM>::sync();
-        team_column_product<TEAM>(W, A, col, np, ld, false);                 // (V M)[:, c0]
-        Team<TEAM>::sync();
-        team_store_column<TEAM>(W, col, np, ld);
-        }
+            Team<TEAM>::sync();
+            team_store_column<TEAM>(A, col, np, ld);
+            Team<TEAM>::sync();
+            team_column_product<TEAM>(W, A, col, np, ld, false);                 // (V M)[:, c0]
+            Team<TEAM>::sync();
+            team_store_column<TEAM>(W, col, np, ld);
+            }
+        };
+        orthonormalise();
         // A <- W^H H W (exactly Hermitian); returns ||H||_F.
         auto project = [&]() {
             const double f = team_load_hermitian<TEAM>(A, h_in + b * h_stride, nw, np, ld, red);   // A <- H
@@ -815,15 +835,18 @@ __global__ void __launch_bounds__(TEAM == 128 ? 128 : 64, TEAM == 32 ? 1 : (TEAM
         // square the off-diagonal ratios, after which the strict completion (2^-26) normally holds
         // without any sweep; the sweeps remain the fallback of either bound.
         bool loose = false;
-        if (converge && team_first_order_completion<TEAM>(A, W, np, ld, dnew, 1.220703125e-04)) {
+        double *cred = converge ? red : nullptr, norm2 = 0.0;
+        if (converge && team_first_order_completion<TEAM>(A, W, np, ld, dnew, 1.220703125e-04, cred, norm2)) {
             loose = true;
+            if (norm2 > COMPLETION_LOOSE2) orthonormalise();
             project();
         }
         for (int sweep = 0; sweep < (converge ? WNLQG_JACOBI_MAX_SWEEPS : 1); ++sweep) {
             const double off = team_offdiag2<TEAM>(A, np, ld, red);
             if (sqrt(off) <= (converge ? tol * np : fro * 1.0e-13)) break;
             if ((converge ? (sweep > 0 || loose) : sweep == 0) &&
-                team_first_order_completion<TEAM>(A, W, np, ld, dnew, converge ? 1.4901161193847656e-08 : 1.220703125e-04))
+                team_first_order_completion<TEAM>(A, W, np, ld, dnew, converge ? 1.4901161193847656e-08 : 1.220703125e-04,
+                                                  cred, norm2))
                 break;
             if (!team_jacobi_sweep<double, TEAM>(A, W, np, ld, tol, rot_s, rot_c)) break;
         }
@@ -1000,7 +1023,7 @@ struct RefineCtaSmem {
 // FP64 tensor cores): on success W <- W (I + E) (Wc and Tc swap roles) and A's diagonal holds the
 // second-order eigenvalues.  dnew: np doubles of shared scratch.
 WNLQG_D bool cta_first_order_completion(double2 *A, double2 *&Wc, double2 *&Tc, int np, int ld, double *dnew,
-                                        double tau) {
+                                        double tau, double *red, double &norm2) {
     const int tid = threadIdx.x;
     int bad = 0;
     for (int e = tid; e < np * np; e += blockDim.x) {
@@ -1021,17 +1044,30 @@ WNLQG_D bool cta_first_order_completion(double2 *A, double2 *&Wc, double2 *&Tc, 
         dnew[j] = dj + s;
     }
     __syncthreads();
+    double local = 0.0;
     for (int e = tid; e < np * np; e += blockDim.x) {
         const int i = e % np, j = e / np;
         const double2 a = A[i + ld * j];
         if (i == j || (a.x == 0.0 && a.y == 0.0)) continue;
         const double g = A[j + ld * j].x - A[i + ld * i].x;
-        A[i + ld * j] = make_double2(a.x / g, a.y / g);
+        const double2 ej = make_double2(a.x / g, a.y / g);
+        local += ej.x * ej.x + ej.y * ej.y;
+        A[i + ld * j] = ej;
+    }
+    if (red) {
+        for (int o = 16; o > 0; o >>= 1) local += __shfl_xor_sync(0xffffffffu, local, o);
+        if ((tid & 31) == 0) red[tid >> 5] = local;
     }
     __syncthreads();
+    bool second = tau > 1.4901161193847656e-08;
+    if (red) {
+        norm2 = 0.0;
+        for (int w = 0; w < (int)(blockDim.x >> 5); ++w) norm2 += red[w];
+        second = second || norm2 > COMPLETION_STRICT2;
+    }
     for (int i = tid; i < np; i += blockDim.x) A[i + ld * i] = make_double2(1.0, 0.0);
     __syncthreads();
-    if (tau > 1.4901161193847656e-08) {                      // A <- ((I + E)^2 + I) / 2
+    if (second) {                                            // A <- ((I + E)^2 + I) / 2
         dmma_product<0>(A, A, Tc, np, ld);
         __syncthreads();
         for (int e = tid; e < np * np; e += blockDim.x) {
@@ -1083,21 +1119,25 @@ __global__ void __launch_bounds__(512, 1) eigh_refine_f64_cta_kernel(const doubl
             Wc[i + ld * j] = to_c64(vi[i + np * j]);
         }
         __syncthreads();
-        dmma_product<1>(Wc, Wc, Tc, np, ld);                 // T = W^H W
-        __syncthreads();
-        for (int i = tid; i < np; i += blockDim.x) Tc[i + ld * i].x -= 1.0;   // E = W^H W - I
-        __syncthreads();
-        dmma_product<0>(Tc, Tc, A, np, ld);                  // A = E^2
-        __syncthreads();
-        for (int e = tid; e < np * np; e += blockDim.x) {    // A = M = I - E/2 + 3 E^2 / 8
-            const int i = e % np, j = e / np, o = i + ld * j;
-            const double2 ev = Tc[o], e2 = A[o];
-            A[o] = make_double2((i == j ? 1.0 : 0.0) - 0.5 * ev.x + 0.375 * e2.x, -0.5 * ev.y + 0.375 * e2.y);
-        }
-        __syncthreads();
-        dmma_product<0>(Wc, A, Tc, np, ld);                  // T = W M
-        __syncthreads();
-        { double2 *x = Wc; Wc = Tc; Tc = x; }                // W <- W M
+        // W <- W (I - E/2 + 3 E^2 / 8), E = W^H W - I.
+        auto orthonormalise = [&]() {
+            dmma_product<1>(Wc, Wc, Tc, np, ld);                 // T = W^H W
+            __syncthreads();
+            for (int i = tid; i < np; i += blockDim.x) Tc[i + ld * i].x -= 1.0;   // E = W^H W - I
+            __syncthreads();
+            dmma_product<0>(Tc, Tc, A, np, ld);                  // A = E^2
+            __syncthreads();
+            for (int e = tid; e < np * np; e += blockDim.x) {    // A = M = I - E/2 + 3 E^2 / 8
+                const int i = e % np, j = e / np, o = i + ld * j;
+                const double2 ev = Tc[o], e2 = A[o];
+                A[o] = make_double2((i == j ? 1.0 : 0.0) - 0.5 * ev.x + 0.375 * e2.x, -0.5 * ev.y + 0.375 * e2.y);
+            }
+            __syncthreads();
+            dmma_product<0>(Wc, A, Tc, np, ld);                  // T = W M
+            __syncthreads();
+            { double2 *x = Wc; Wc = Tc; Tc = x; }                // W <- W M
+        };
+        orthonormalise();
         // A <- W^H H W (exactly Hermitian), H from its upper triangle, zero-padded; returns ||H||_F.
         const double2 *h = h_in + b * h_stride;
         auto project = [&]() {
@@ -1135,8 +1175,11 @@ __global__ void __launch_bounds__(512, 1) eigh_refine_f64_cta_kernel(const doubl
         // FP64 path: the loose completion and a fresh projection before the strict one, as in the team
         // kernel; the sweeps are the fallback of either bound.
         bool loose = false;
-        if (converge && cta_first_order_completion(A, Wc, Tc, np, ld, reinterpret_cast<double *>(rot_s), 1.220703125e-04)) {
+        double *cred = converge ? red : nullptr, norm2 = 0.0;
+        if (converge && cta_first_order_completion(A, Wc, Tc, np, ld, reinterpret_cast<double *>(rot_s), 1.220703125e-04,
+                                                   cred, norm2)) {
             loose = true;
+            if (norm2 > COMPLETION_LOOSE2) orthonormalise();
             project();
         }
         for (int sweep = 0; sweep < (converge ? WNLQG_JACOBI_MAX_SWEEPS : 1); ++sweep) {
@@ -1144,7 +1187,7 @@ __global__ void __launch_bounds__(512, 1) eigh_refine_f64_cta_kernel(const doubl
             if (off <= (converge ? tol * np : fro * 1.0e-13)) break;
             if ((converge ? (sweep > 0 || loose) : sweep == 0) &&
                 cta_first_order_completion(A, Wc, Tc, np, ld, reinterpret_cast<double *>(rot_s),
-                                           converge ? 1.4901161193847656e-08 : 1.220703125e-04))
+                                           converge ? 1.4901161193847656e-08 : 1.220703125e-04, cred, norm2))
                 break;
             if (tid == 0) rot_flag = 0;
             __syncthreads();
