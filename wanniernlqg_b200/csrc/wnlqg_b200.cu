@@ -216,8 +216,6 @@ struct wnlqg_plan {
     size_t osort_bytes = 0;
     cudaStream_t stream = nullptr;
     std::vector<cudaEvent_t> events;
-    void *h_stage = nullptr;                  // pinned staging of copy_to_host (two halves), lazily allocated
-    cudaEvent_t h_stage_ev[2] = {nullptr, nullptr};
     size_t timing_batches = 0;
     int64_t launches = 0;
     bool timing_valid = false;
@@ -1341,9 +1339,6 @@ wnlqg_status wnlqg_b200_plan_destroy(wnlqg_plan *pl) {
                       (void *)pl->d_fd_tiles})
         if (ptr) cudaFree(ptr);
     for (cudaEvent_t ev : pl->events) cudaEventDestroy(ev);
-    for (cudaEvent_t ev : pl->h_stage_ev)
-        if (ev) cudaEventDestroy(ev);
-    if (pl->h_stage) cudaFreeHost(pl->h_stage);
     if (pl->stream) cudaStreamDestroy(pl->stream);
     delete pl;
     return WNLQG_OK;
@@ -2543,47 +2538,6 @@ __global__ void transpose_vectors_kernel(const double2 *__restrict__ U, int64_t 
     out[b * nn + (int64_t)(r % nw) * nw + r / nw] = U[e];
 }
 
-// Device memory to pageable host memory on the plan's stream, complete on return: in chunks through two
-// pinned halves kept by the plan, the host copying one chunk out while the next is on its way (the
-// driver's own staging of a pageable destination took 1.2 ms for 9 MB of fresh memory; 601 points of 31
-// orbitals, spectrum and vectors, 2.9 -> 1.3 ms with this and the device transposition).
-// Without pinned memory the plain copy.
-wnlqg_status copy_to_host(wnlqg_plan *pl, void *dst, const void *src, size_t bytes) {
-    constexpr size_t half = (size_t)2 << 20;
-    if (!pl->h_stage && bytes > (size_t)(64 << 10)) {
-        if (cudaMallocHost(&pl->h_stage, 2 * half) != cudaSuccess) {
-            cudaGetLastError();
-            pl->h_stage = nullptr;
-        }
-        for (int i = 0; i < 2 && pl->h_stage; ++i)
-            if (!pl->h_stage_ev[i]) WNLQG_CUDA(cudaEventCreateWithFlags(&pl->h_stage_ev[i], cudaEventDisableTiming));
-    }
-    if (!pl->h_stage || bytes <= (size_t)(64 << 10)) {
-        WNLQG_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, pl->stream));
-        WNLQG_CUDA(cudaStreamSynchronize(pl->stream));
-        return WNLQG_OK;
-    }
-    unsigned char *stage = static_cast<unsigned char *>(pl->h_stage);
-    const size_t chunks = (bytes + half - 1) / half;
-    auto issue = [&](size_t c) -> wnlqg_status {
-        const size_t off = c * half, len = std::min(half, bytes - off);
-        WNLQG_CUDA(cudaMemcpyAsync(stage + (c & 1) * half, static_cast<const unsigned char *>(src) + off, len,
-                                   cudaMemcpyDeviceToHost, pl->stream));
-        WNLQG_CUDA(cudaEventRecord(pl->h_stage_ev[c & 1], pl->stream));
-        return WNLQG_OK;
-    };
-    wnlqg_status st;
-    for (size_t c = 0; c < std::min<size_t>(2, chunks); ++c)
-        if ((st = issue(c)) != WNLQG_OK) return st;
-    for (size_t c = 0; c < chunks; ++c) {
-        const size_t off = c * half, len = std::min(half, bytes - off);
-        WNLQG_CUDA(cudaEventSynchronize(pl->h_stage_ev[c & 1]));
-        std::memcpy(static_cast<unsigned char *>(dst) + off, stage + (c & 1) * half, len);
-        if (c + 2 < chunks && (st = issue(c + 2)) != WNLQG_OK) return st;
-    }
-    return WNLQG_OK;
-}
-
 wnlqg_status eval_spectrum(wnlqg_plan *pl, const double *kpoints, int64_t n, double *energies, double *eigenvectors,
                            bool rows) {
     wnlqg_status st = check_plan(pl);
@@ -2605,14 +2559,17 @@ wnlqg_status eval_spectrum(wnlqg_plan *pl, const double *kpoints, int64_t n, dou
         if (eigenvectors) {
             const double2 *src = pl->d_U;
             if (rows) {
-                // The channels are spent once the vectors exist: their buffer takes the transposes.
+                // The channels are spent once the vectors exist: their buffer takes the transposes.  601 points
+                // of 31 orbitals, row-major vectors: 2.9 ms with the transposition on the host, 1.2 with this.
+                // The copy is the plain one: pinned halves with the host copying a chunk out while the next
+                // is on its way took 1.3, and their allocation 1.4 to 3 ms more in a plan's first call.
                 transpose_vectors_kernel<<<(unsigned)((nb * pl->nn + 255) / 256), 256, 0, pl->stream>>>(pl->d_U, nb, pl->nw,
                                                                                                      pl->d_xw);
                 WNLQG_CUDA(cudaGetLastError());
                 src = pl->d_xw;
             }
-            if ((st = copy_to_host(pl, eigenvectors + 2 * s * pl->nn, src, (size_t)nb * pl->nn * sizeof(double2))) != WNLQG_OK)
-                return st;
+            WNLQG_CUDA(cudaMemcpyAsync(eigenvectors + 2 * s * pl->nn, src, (size_t)nb * pl->nn * sizeof(double2),
+                                       cudaMemcpyDeviceToHost, pl->stream));
         }
     }
     WNLQG_CUDA(cudaStreamSynchronize(pl->stream));
