@@ -17,7 +17,7 @@
 //      scratch (nine nw x nw matrices).
 //   3. Active pairs (|f_n - f_m| >= 1e-10) are compacted; per pair and component the seven
 //      k-local coefficients (first ... fifth, the two three-band sums) go to global scratch.
-//   4. Frequency contraction: a thread owns one photon energy and SHG_CB components and streams
+//   4. Frequency contraction: a thread owns one photon energy and two or three components and streams
 //      the pair list once, evaluating the three resonance kernels per pair; the five pair terms of
 //      both quantities follow from nine accumulators per component plus three frequency-independent
 //      sums.
@@ -28,7 +28,6 @@
 #include "response.cuh"
 
 #define SHG_MAX_COMPONENTS 81
-#define SHG_CB 2                         // components per thread in the frequency contraction
 #define SHG_KB_EV 8.617333262145e-5      // RESPONSE_KB_EV of the reference's SHG occupations
 
 struct ShgParams {
@@ -150,7 +149,10 @@ WNLQG_D void shg_emit(const ShgParams &p, int64_t b, int64_t idx, double2 v, dou
     }
 }
 
-// Frequency contraction for one thread: photon energy `om`, components c0 .. c0+SHG_CB-1.  The pair
+// Components per thread in the frequency contraction.
+WNLQG_HD constexpr int shg_components(bool pair) { return pair ? 2 : 3; }
+
+// Frequency contraction for one thread: photon energy `om`, components c0 .. c0 + CB - 1.  The pair
 // factors go on the three resonances once per pair and energy, so that a component costs thirteen
 // complex multiply-adds:
 //   P1 = sum fo inv (2 first d2 + second d1)      P2 = sum fo inv third (d1 - 4 d2)
@@ -158,7 +160,7 @@ WNLQG_D void shg_emit(const ShgParams &p, int64_t b, int64_t idx, double2 v, dou
 //   P5 = sum fo fifth d1                          P6 = sum fo (first d2 + second d1)
 //   P7 = sum fo third (d1 - 2 d2)                 P8 = sum fo diff (tf d2 - to dn)
 //   P9 = sum fo fourth d1
-template <bool GAUSS>
+template <bool GAUSS, int CB>
 WNLQG_D void shg_contract(const ShgParams &p, const double2 *__restrict__ coef, const double *__restrict__ pinfo,
                           int npairs, double om, int c0, double2 (*acc)[9]) {
     const double w = p.width, w2 = w * w, gpref = 1.7724538509055160273 / w;
@@ -174,7 +176,7 @@ WNLQG_D void shg_contract(const ShgParams &p, const double2 *__restrict__ coef, 
         const double2 oo2 = cscale(d2, 2.0 * fo), on = cscale(dn, fo), e2 = cscale(d2, fd), en = cscale(dn, -fd);
         const double2 i3 = make_double2(fma(-2.0, i2.x, i1.x), fma(-2.0, i2.y, i1.y)), o3 = csub(o1, oo2);
 #pragma unroll
-        for (int j = 0; j < SHG_CB; ++j) {
+        for (int j = 0; j < CB; ++j) {
             const int c = c0 + j;
             if (c >= nc) break;
             const double2 *cf = coef + ((int64_t)q * nc + c) * 7;
@@ -193,13 +195,17 @@ WNLQG_D void shg_contract(const ShgParams &p, const double2 *__restrict__ coef, 
     }
 }
 
-// GW: matrices in the per-CTA global working set (large nw); else dynamic shared memory.  Two CTAs per SM
-// where shared memory allows (128 registers, two components per thread): the serial parts of one
-// point then overlap the other's.  With the pair factors on the resonances, the refined reciprocal
-// instead of IEEE quotients and the low-frequency sums by warps, second harmonic spectra (256
-// energies) of 16 orbitals and two components on a 12^3 mesh take 2.82 -> 2.49 ms.
-template <bool GW>
-__global__ void __launch_bounds__(256, 2) shg_kernel(ShgParams p) {
+// GW: matrices in the per-CTA global working set (large nw); else dynamic shared memory.
+// PAIR: two CTAs per SM, at 128 registers and two components per thread, so that the serial parts of
+// one point overlap the other's; else one, at up to 255 registers and three components, which always
+// is the form of a global working set (80 orbitals, 3 components, 256 energies: 26.0 ms with the
+// products scaled one by one, 29.3 at 128 registers and two components, 24.0 so) and the one of shared
+// memory above 22 orbitals.  With the pair factors on the resonances, the refined reciprocal instead of
+// IEEE quotients and the low-frequency sums by warps, 1184 points of 16 orbitals, two components and
+// 128 energies take 1.97 -> 1.54 ms (PAIR), 592 of 26 orbitals 3.07 -> 2.53.
+template <bool GW, bool PAIR>
+__global__ void __launch_bounds__(256, PAIR ? 2 : 1) shg_kernel(ShgParams p) {
+    constexpr int CB = shg_components(PAIR);
     extern __shared__ __align__(16) unsigned char smem_dyn[];
     unsigned char *sm;
     if constexpr (GW) sm = p.gscratch + (int64_t)blockIdx.x * p.gscratch_stride;
@@ -415,21 +421,21 @@ __global__ void __launch_bounds__(256, 2) shg_kernel(ShgParams p) {
         __syncthreads();
 
         // Stage 4: pair terms 1-5 of both quantities.
-        const int nchunks = (nc + SHG_CB - 1) / SHG_CB;
+        const int nchunks = (nc + CB - 1) / CB;
         for (int it = threadIdx.x; it < p.nom * nchunks; it += blockDim.x) {
-            const int w = it % p.nom, c0 = (it / p.nom) * SHG_CB;
+            const int w = it % p.nom, c0 = (it / p.nom) * CB;
             const double om = p.omegas[w];
-            double2 acc[SHG_CB][9];
+            double2 acc[CB][9];
 #pragma unroll
-            for (int j = 0; j < SHG_CB; ++j)
+            for (int j = 0; j < CB; ++j)
 #pragma unroll
                 for (int t = 0; t < 9; ++t) acc[j][t] = make_double2(0.0, 0.0);
-            if (p.gaussian) shg_contract<true>(p, coef, pinfo, npairs, om, c0, acc);
-            else shg_contract<false>(p, coef, pinfo, npairs, om, c0, acc);
+            if (p.gaussian) shg_contract<true, CB>(p, coef, pinfo, npairs, om, c0, acc);
+            else shg_contract<false, CB>(p, coef, pinfo, npairs, om, c0, acc);
             if (p.mode == 0 && npairs == 0) continue;
             const double low = shg_principal(om, p.low_width);
 #pragma unroll
-            for (int j = 0; j < SHG_CB; ++j) {
+            for (int j = 0; j < CB; ++j) {
                 const int c = c0 + j;
                 if (c >= nc) break;
                 const double2 s1 = sS[3 * c], s2 = sS[3 * c + 1], s4 = sS[3 * c + 2];

@@ -122,7 +122,8 @@ struct wnlqg_plan {
     double *d_E = nullptr, *d_kpts = nullptr, *d_omegas = nullptr, *d_partials = nullptr, *d_weights = nullptr;
     double *d_mus = nullptr;
     int64_t *d_kidx = nullptr;
-    int partial_slots = 0;
+    int partial_slots = 0;                    // partial sums' slots: allocated, needed beside the second
+    int other_slots = 0, call_slots = 0;      // harmonic's, and of the call in progress (begin_call)
     // Staged mesh Fourier: R grouping (device) and lazily sized Y/Z workspaces.
     int P12 = 0, P1 = 0;
     int *d_groups = nullptr;        // q12_start | q12_ridx | q12_r2 | q1_start | q1_q12 | q1_r1
@@ -140,6 +141,8 @@ struct wnlqg_plan {
     double2 *d_shg_scratch = nullptr;
     unsigned char *d_shg_gscratch = nullptr;
     bool shg_global = false;
+    bool shg_pair = false;                    // two CTAs per SM fit (shg_takes_pairs says when they pay)
+    bool shg_pair_now = false;                // and the call in progress takes them (begin_call)
     // Tensor-core Fourier for arbitrary k-points: Ozaki slices of the phases (A, per batch) and of
     // the channel tiles (B, built once), tcgen05 kind::i8 GEMM.  tc_slices == 0: FP64 CUDA cores.
     int tc_slices = 0;
@@ -566,6 +569,32 @@ wnlqg_status build_passes(wnlqg_plan *pl, int sm_count, size_t smem_limit) {
 
 // Second-harmonic launches: parameters per SHG response, shared-memory size, grid and the per-CTA
 // global scratch (G matrices, pair coefficients, pair data).
+// The second-harmonic kernel's instantiation.
+const void *shg_function(bool global, bool pair) {
+    if (global) return (const void *)shg_kernel<true, false>;
+    return pair ? (const void *)shg_kernel<false, true> : (const void *)shg_kernel<false, false>;
+}
+
+// Whether a launch takes the form with two CTAs per SM, where shared memory allows it.  Two conditions.
+//   - The contraction, in passes of 256 threads over the energies and component chunks: the narrower
+//     chunks of that form may need more passes, and each evaluates the resonances again.  1184 points
+//     of 22 orbitals, one CTA -> two: 3.76 -> 3.11 ms (3 components, 48 energies: 1 pass either way),
+//     11.48 -> 10.95 (6, 400: 4 and 5), 7.56 -> 7.85 (6, 256: 2 and 3), 4.29 -> 4.56 (3, 256: 1 and 2; 5.16 ->
+//     6.12 with the Gaussian's exponentials).  Up to 8 orbitals the other steps outweigh that: 0.72 -> 0.63
+//     at 4 (3, 256).
+//   - Rounds of points over the SMs: a round of two points takes 1.4 to 1.7 times one of one point, least
+//     for few orbitals and energies.  300 points, 3 rounds -> 2: 16 orbitals 0.86 -> 1.08 ms (2 components,
+//     256 energies), 4 orbitals 0.29 -> 0.25 (1, 48).
+bool shg_takes_pairs(const ShgParams &p, int64_t nb, int sm_count) {
+    auto passes = [&](bool pair) {
+        const int cb = shg_components(pair);
+        return ((int64_t)p.nom * ((p.nc + cb - 1) / cb) + 255) / 256;
+    };
+    const int64_t ones = (nb + sm_count - 1) / sm_count, pairs = (nb + 2 * sm_count - 1) / (2 * sm_count);
+    const bool light = p.nw <= 12 && (int64_t)p.nc * p.nom <= 256;
+    return (p.nw <= 8 || 5 * passes(true) <= 7 * passes(false)) && (light ? 15 : 17) * pairs <= 10 * ones;
+}
+
 wnlqg_status build_shg(wnlqg_plan *pl, int sm_count, size_t smem_limit) {
     const wnlqg_task_desc &t = pl->task;
     int64_t off = 0;
@@ -614,23 +643,29 @@ wnlqg_status build_shg(wnlqg_plan *pl, int sm_count, size_t smem_limit) {
     const bool shg_global = shg_bytes > smem_limit;   // large nw: matrices in a per-CTA global working set
     pl->shg_smem = shg_global ? 0 : shg_bytes;
     pl->shg_global = shg_global;
-    const void *shg_fn = shg_global ? (const void *)shg_kernel<true> : (const void *)shg_kernel<false>;
+    const void *shg_fn = shg_function(shg_global, false);
     cudaError_t e = allow_dynamic_smem(shg_fn, (int)smem_limit);
+    if (e == cudaSuccess && !shg_global) e = allow_dynamic_smem(shg_function(false, true), (int)smem_limit);
     if (e != cudaSuccess) return fail(WNLQG_ERR_CUDA, std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(e));
-    int per_sm = 0;
+    int per_sm = 0, pair_per_sm = 0;
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, shg_fn, 256, pl->shg_smem);
+    if (e == cudaSuccess && !shg_global)
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&pair_per_sm, shg_function(false, true), 256, pl->shg_smem);
     if (e != cudaSuccess) return fail(WNLQG_ERR_CUDA, std::string("occupancy query: ") + cudaGetErrorString(e));
     if (per_sm < 1) return fail(WNLQG_ERR_UNSUPPORTED, "second-harmonic kernel cannot be resident with its shared memory");
     pl->shg_grid = sm_count * per_sm;
+    pl->shg_pair = pair_per_sm >= 2;
     // A global working set is allocated for up to two CTAs per SM; one CTA per SM is the default
     // (measured at 64 orbitals: the L2-resident half grid is slower), the autotuner may change it.
-    pl->shg_grid_alloc = shg_global ? std::max(pl->shg_grid, 2 * sm_count) : pl->shg_grid;
+    pl->shg_grid_alloc = shg_global || pl->shg_pair ? std::max(pl->shg_grid, 2 * sm_count) : pl->shg_grid;
     if (shg_global) {
         pl->shg_grid_l2 = l2_resident_grid(pl->shg_grid, (int64_t)shg_bytes, sm_count);
         pl->shg_grid = sm_count;
     }
-    if (const char *g = std::getenv("WNLQG_B200_SHG_GRID"))
+    if (const char *g = std::getenv("WNLQG_B200_SHG_GRID")) {
         pl->shg_grid = std::max(1, std::min(pl->shg_grid_alloc, std::atoi(g)));
+        pl->shg_pair = false;
+    }
     const int64_t stride = ShgSmem::scratch_entries(pl->nw, max_nc);
     for (ShgParams &p : pl->shg) p.scratch_stride = stride;
     e = cudaMalloc(&pl->d_shg_scratch, (size_t)pl->shg_grid_alloc * stride * sizeof(double2));
@@ -1176,8 +1211,10 @@ wnlqg_status run_passes(wnlqg_plan *pl, int64_t nb, int mode, double scale, int6
         p.out_perm = out_perm;
         p.scratch = pl->d_shg_scratch;
         p.gscratch = pl->d_shg_gscratch;
-        if (pl->shg_global) shg_kernel<true><<<pl->shg_grid, 256, pl->shg_smem, pl->stream>>>(p);
-        else shg_kernel<false><<<pl->shg_grid, 256, pl->shg_smem, pl->stream>>>(p);
+        void *args[] = {(void *)&p};
+        WNLQG_CUDA(cudaLaunchKernel(shg_function(pl->shg_global, pl->shg_pair_now),
+                                    dim3(pl->shg_pair_now ? 2 * pl->sm_count : pl->shg_grid), dim3(256), args,
+                                    pl->shg_smem, pl->stream));
         pl->launches += 1;
     }
     WNLQG_CUDA(cudaGetLastError());
@@ -2160,8 +2197,9 @@ wnlqg_status wnlqg_b200_plan_create(wnlqg_model *model, const wnlqg_task_desc *t
     for (const Pass &ps : pl->passes)
         pl->partial_slots = std::max(pl->partial_slots, std::max(ps.global ? std::max(ps.grid, 2 * sm_count) : ps.grid,
                                                                    ps.grid_wide));
-    pl->partial_slots = std::max(pl->partial_slots, pl->shg_grid_alloc);
     pl->partial_slots = std::max(pl->partial_slots, pl->bcda_grid);
+    pl->other_slots = std::max(pl->partial_slots, sm_count);   // the Fermi-sea dipole's grid is at most sm_count
+    pl->partial_slots = std::max(pl->partial_slots, pl->shg_grid_alloc);
     if ((st = alloc((void **)&pl->d_partials, (size_t)pl->partial_slots * vc * 4 * sizeof(double))) != WNLQG_OK)
         return bail(st);
     *out_plan = pl;
@@ -2191,11 +2229,28 @@ wnlqg_status order_batch(wnlqg_plan *pl, const double *k, const double *w, int64
     return WNLQG_OK;
 }
 
+// The form of the second-harmonic kernel and the partial sums' slots for a call over n points.
+void begin_call(wnlqg_plan *pl, int64_t n) {
+    pl->shg_pair_now = false;
+    if (pl->shg_pair)
+        for (const ShgParams &p : pl->shg)
+            pl->shg_pair_now |= shg_takes_pairs(p, std::min(n, pl->max_batch), pl->sm_count);
+    const int shg_slots = pl->shg.empty() ? 0 : (pl->shg_pair_now ? 2 * pl->sm_count : pl->shg_grid);
+    pl->call_slots = std::min(pl->partial_slots, std::max(pl->other_slots, shg_slots));
+}
+
+// The same for a call that sums: the slots it uses, zeroed.
+wnlqg_status begin_sums(wnlqg_plan *pl, int64_t n) {
+    begin_call(pl, n);
+    WNLQG_CUDA(cudaMemsetAsync(pl->d_partials, 0, (size_t)pl->call_slots * pl->vc * 4 * sizeof(double), pl->stream));
+    return WNLQG_OK;
+}
+
 // The plan's partial sums, summed over their slots into out (device, value-count complex values).
 wnlqg_status launch_reduce(wnlqg_plan *pl, double2 *out) {
     const int64_t vx = reduce_values_per_block(pl->vc);
     reduce_partials_kernel<<<(unsigned)std::max<int64_t>(1, (pl->vc + vx - 1) / vx), REDUCE_THREADS, 0, pl->stream>>>(
-        pl->d_partials, pl->partial_slots, pl->vc, out);
+        pl->d_partials, pl->call_slots, pl->vc, out);
     pl->launches += 1;
     WNLQG_CUDA(cudaGetLastError());
     return WNLQG_OK;
@@ -2227,7 +2282,7 @@ wnlqg_status enqueue_mesh(wnlqg_plan *pl, const int64_t mesh[3], int64_t k_begin
     const int64_t nk = mesh[0] * mesh[1] * mesh[2];
     if ((st = record_event(pl, 0)) != WNLQG_OK) return st;
     pl->launches = 0;
-    WNLQG_CUDA(cudaMemsetAsync(pl->d_partials, 0, (size_t)pl->partial_slots * pl->vc * 4 * sizeof(double), pl->stream));
+    if ((st = begin_sums(pl, k_end - k_begin)) != WNLQG_OK) return st;
     const double scale = 1.0 / (double)nk;
     size_t nbatch = 0;
     for (int64_t s = k_begin; s < k_end; s += pl->max_batch, ++nbatch) {
@@ -2300,7 +2355,7 @@ wnlqg_status enqueue_points_weighted(wnlqg_plan *pl, const double *kpoints_devic
     wnlqg_status st;
     if ((st = record_event(pl, 0)) != WNLQG_OK) return st;
     pl->launches = 0;
-    WNLQG_CUDA(cudaMemsetAsync(pl->d_partials, 0, (size_t)pl->partial_slots * pl->vc * 4 * sizeof(double), pl->stream));
+    if ((st = begin_sums(pl, n)) != WNLQG_OK) return st;
     size_t nbatch = 0;
     for (int64_t s = 0; s < n; s += pl->max_batch, ++nbatch) {
         const int64_t nb = std::min(pl->max_batch, n - s);
@@ -2421,6 +2476,7 @@ wnlqg_status wnlqg_b200_eval_points(wnlqg_plan *pl, const double *kpoints, int64
     if (!finite_array(kpoints, 3 * (size_t)n)) return fail(WNLQG_ERR_NONFINITE, "k-points must be finite");
     WNLQG_CUDA(cudaSetDevice(pl->model->device));
     pl->launches = 0;
+    begin_call(pl, n);
     for (int64_t s = 0; s < n; s += pl->max_batch) {
         int64_t nb = std::min(pl->max_batch, n - s);
         WNLQG_CUDA(cudaMemcpyAsync(pl->d_kpts, kpoints + 3 * s, (size_t)nb * 3 * sizeof(double), cudaMemcpyHostToDevice,
@@ -2455,7 +2511,7 @@ wnlqg_status wnlqg_b200_eval_points_weighted(wnlqg_plan *pl, const double *kpoin
         return fail(WNLQG_ERR_NONFINITE, "k-points and weights must be finite");
     WNLQG_CUDA(cudaSetDevice(pl->model->device));
     pl->launches = 0;
-    WNLQG_CUDA(cudaMemsetAsync(pl->d_partials, 0, (size_t)pl->partial_slots * pl->vc * 4 * sizeof(double), pl->stream));
+    if ((st = begin_sums(pl, n)) != WNLQG_OK) return st;
     for (int64_t s = 0; s < n; s += pl->max_batch) {
         int64_t nb = std::min(pl->max_batch, n - s);
         WNLQG_CUDA(cudaMemcpyAsync(pl->d_kpts, kpoints + 3 * s, (size_t)nb * 3 * sizeof(double), cudaMemcpyHostToDevice,
@@ -2494,7 +2550,7 @@ wnlqg_status wnlqg_b200_eval_mesh_weighted(wnlqg_plan *pl, const int64_t mesh[3]
     if (!finite_array(weights, (size_t)n)) return fail(WNLQG_ERR_NONFINITE, "weights must be finite");
     WNLQG_CUDA(cudaSetDevice(pl->model->device));
     pl->launches = 0;
-    WNLQG_CUDA(cudaMemsetAsync(pl->d_partials, 0, (size_t)pl->partial_slots * pl->vc * 4 * sizeof(double), pl->stream));
+    if ((st = begin_sums(pl, n)) != WNLQG_OK) return st;
     for (int64_t s = 0; s < n; s += pl->max_batch) {
         const int64_t nb = std::min(pl->max_batch, n - s);
         bool contiguous = true;
