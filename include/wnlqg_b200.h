@@ -363,7 +363,9 @@ WNLQG_API wnlqg_status wnlqg_b200_graph_destroy(wnlqg_graph *graph);
  * the partial sums: on the FP64 path they may change results in the last bits; on the mixed path
  * they also change which neighbour each point's FP32 eigensolve warm-starts from, so results
  * change within the mixed path's accuracy (about 1e-6 relative).  Times are CUDA-event milliseconds of the second of two runs; -1 = not a
- * candidate; 0 in a choice = not tunable for this plan. */
+ * candidate; 0 in a choice = not tunable for this plan.  Up to 16 orbitals on the FP64 path the
+ * eigensolver is one kernel without a team or a warm start: its one time is given for each of those
+ * candidates, and the choices are the plan's settings. */
 typedef struct wnlqg_autotune_report {
     int32_t eigh_team;             /* chosen threads per matrix (32, 64, 128), 0 = fixed variant */
     int32_t energies_per_thread;   /* chosen contraction tile (1, 2, 4), 0 = no energy axis */

@@ -2885,8 +2885,8 @@ wnlqg_status wnlqg_b200_graph_destroy(wnlqg_graph *graph) {
 }  // extern "C"
 
 // ---------------------------------------------------------------------------------------------
-// Autotuner: per orbital count, the eigensolver team (threads per matrix of the FP32 Jacobi and
-// FP64 refinement stages, orthogonal models up to 32 orbitals) and the contraction tile (photon
+// Autotuner: per orbital count, the eigensolver team (threads per matrix of the FP64 refinement and,
+// on the mixed path, the FP32 Jacobi; up to 32 orbitals) and the contraction tile (photon
 // energies per thread) measured on the caller's own mesh block; the fastest of each is kept in
 // the plan and remembered for the process (device, orbitals, precision, geometry, energies,
 // values).  Every candidate is a configuration the library runs anyway.
@@ -2990,7 +2990,15 @@ extern "C" wnlqg_status wnlqg_b200_plan_autotune(wnlqg_plan *pl, const int64_t m
         pl->eigh_grid = rep.eigh_grid;
     }
     const int teams[3] = {32, 64, 128}, ombs[3] = {1, 2, 4};
-    if (pl->warp_eigh) {
+    if (pl->small_f64) {
+        // One kernel reads neither the team nor the start: one time stands for every candidate, and the
+        // plan keeps its settings.
+        double r = 0;
+        if ((st = tune_measure(pl, mesh, k_begin, k_end, &rep.eigh_ms[0], &r)) != WNLQG_OK) return st;
+        rep.eigh_ms[1] = rep.eigh_ms[2] = rep.start_ms[0] = rep.start_ms[1] = rep.eigh_ms[0];
+        rep.eigh_team = pl->eigh_team;
+        rep.warm_start = pl->warm_mode;
+    } else if (pl->warp_eigh) {
         const int start = pl->eigh_team;
         int best = start;
         double best_ms = std::numeric_limits<double>::infinity(), r = 0;
@@ -3005,7 +3013,7 @@ extern "C" wnlqg_status wnlqg_b200_plan_autotune(wnlqg_plan *pl, const int64_t m
         apply_team(pl, best);
         rep.eigh_team = best;
     }
-    if (pl->warp_eigh || pl->cta_mixed) {
+    if ((pl->warp_eigh && !pl->small_f64) || pl->cta_mixed) {
         const int start = pl->warm_mode;
         double r = 0;
         for (int w = 0; w < 2; ++w) {
