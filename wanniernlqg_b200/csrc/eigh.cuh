@@ -1385,11 +1385,11 @@ __global__ void generalized_eigh_kernel(const double2 *__restrict__ h_in, const 
 }
 
 // ---------------------------------------------------------------------------------------------
-// Mixed-precision generalised eigensolve (nonorthogonal models on the mixed path): the FP64
-// Cholesky S = L L^H and reduction C = L^-1 H L^-H (cholesky_reduce_kernel, the same arithmetic
-// as generalized_eigh_kernel), the orthogonal mixed-precision stages on C (FP32 Jacobi, FP64
-// refinement, ascending order and canonical phases of C's eigenvectors V), then U = L^-H V and
-// the canonical phase rule on U (gen_back_substitute_kernel), so U^H S U = I.
+// Generalised eigensolve of nonorthogonal models in the plan's precision: the FP64 Cholesky
+// S = L L^H and reduction C = L^-1 H L^-H (cholesky_reduce_kernel, the same arithmetic as
+// generalized_eigh_kernel), the orthogonal eigensolver of that precision on C (ascending order and
+// canonical phases of C's eigenvectors V), then U = L^-H V and the canonical phase rule on U
+// (gen_back_substitute_kernel), so U^H S U = I.
 // ---------------------------------------------------------------------------------------------
 struct GenReduceSmem {
     static __host__ __device__ size_t bytes(int nw) {

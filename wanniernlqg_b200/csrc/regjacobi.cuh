@@ -36,16 +36,11 @@ template <int NP> struct RegGroup {
     }
 };
 
-template <typename T> struct alignas(16) RegRot { T c, sx, sy, pad; };
-
-WNLQG_D float reg_rsqrt(float x) { return rsqrtf(x); }
-WNLQG_D double reg_rsqrt(double x) { return rsqrt(x); }
-WNLQG_D float reg_rcp(float x) { return __frcp_rn(x); }
-WNLQG_D double reg_rcp(double x) { return 1.0 / x; }
+struct alignas(16) RegRot { double c, sx, sy, pad; };
 
 // out = a[sel], 0 <= sel < N, by a tree of selects (static register indices).
-template <int N, typename C> WNLQG_D C reg_select(const C *a, int sel) {
-    C t[N];
+template <int N> WNLQG_D double2 reg_select(const double2 *a, int sel) {
+    double2 t[N];
 #pragma unroll
     for (int j = 0; j < N; ++j) t[j] = a[j];
     int n = N;
@@ -70,10 +65,8 @@ template <int N, typename C> WNLQG_D C reg_select(const C *a, int sel) {
 // One sweep (NP - 1 rounds) of the group's matrix: a, v rows of A and V, d the diagonal element of
 // this lane's index.  Elements with |a_pq| <= tol are left.  rot: 2 x NP / 2 rotations of the group's
 // shared memory.  Slot s holds index s at entry and exit.  Returns whether the group rotated.
-template <typename T, int NP>
-WNLQG_D bool reg_jacobi_sweep(typename cplx_of<T>::type (&a)[NP], typename cplx_of<T>::type (&v)[NP], T &d, T tol,
-                              RegRot<T> *rot) {
-    typedef typename cplx_of<T>::type C;
+template <int NP>
+WNLQG_D bool reg_jacobi_sweep(double2 (&a)[NP], double2 (&v)[NP], double &d, double tol, RegRot *rot) {
     typedef RegGroup<NP> G;
     constexpr int H = NP / 2;
     const int i = G::lane();
@@ -89,36 +82,36 @@ WNLQG_D bool reg_jacobi_sweep(typename cplx_of<T>::type (&a)[NP], typename cplx_
         if (!active) partner = i;
         const bool upper = pos >= H;
         // beta = A[upper index, lower index] from the upper lane's row.
-        const C own = reg_select<H>(a, upper ? ps : 0);
-        C beta;
+        const double2 own = reg_select<H>(a, upper ? ps : 0);
+        double2 beta;
         beta.x = G::from(own.x, partner);
         beta.y = G::from(own.y, partner);
         if (upper) beta = own;
-        const T dp = G::from(d, partner);
-        const T g2 = beta.x * beta.x + beta.y * beta.y;
-        T c = (T)1;
-        C s = czero<C>();   // x' = c x - conj(s) y, y' = s x + c y for the lower slot x and the upper y
+        const double dp = G::from(d, partner);
+        const double g2 = beta.x * beta.x + beta.y * beta.y;
+        double c = 1.0;
+        double2 s = make_double2(0.0, 0.0);   // x' = c x - conj(s) y, y' = s x + c y for the lower slot x and the upper y
         if (active && g2 > tol * tol) {
-            const T ginv = reg_rsqrt(g2);
-            const T theta = (upper ? d - dp : dp - d) * ((T)0.5 * ginv);
-            const T tt = copysign(reg_rcp(fabs(theta) + sqrt(theta * theta + (T)1)), theta);
-            c = reg_rsqrt(tt * tt + (T)1);
-            const T sg = tt * c * ginv;
+            const double ginv = rsqrt(g2);
+            const double theta = (upper ? d - dp : dp - d) * (0.5 * ginv);
+            const double tt = copysign(1.0 / (fabs(theta) + sqrt(theta * theta + 1.0)), theta);
+            c = rsqrt(tt * tt + 1.0);
+            const double sg = tt * c * ginv;
             s.x = sg * beta.x;
             s.y = -sg * beta.y;
-            const T shift = tt * (g2 * ginv);
+            const double shift = tt * (g2 * ginv);
             d += upper ? shift : -shift;
             rotated = true;
         }
-        RegRot<T> *r = rot + (round & 1) * H;
+        RegRot *r = rot + (round & 1) * H;
         if (active && !upper) {
-            RegRot<T> q;
-            q.c = c; q.sx = s.x; q.sy = s.y; q.pad = (T)0;
+            RegRot q;
+            q.c = c; q.sx = s.x; q.sy = s.y; q.pad = 0.0;
             r[pos] = q;
         }
         __syncwarp();
-        auto columns = [&](C &x, C &y, const RegRot<T> &q) {
-            const C x0 = x, y0 = y;
+        auto columns = [&](double2 &x, double2 &y, const RegRot &q) {
+            const double2 x0 = x, y0 = y;
             x.x = fma(-q.sy, y0.y, fma(-q.sx, y0.x, q.c * x0.x));
             x.y = fma(q.sy, y0.x, fma(-q.sx, y0.y, q.c * x0.y));
             y.x = fma(-q.sy, x0.y, fma(q.sx, x0.x, q.c * y0.x));
@@ -126,20 +119,20 @@ WNLQG_D bool reg_jacobi_sweep(typename cplx_of<T>::type (&a)[NP], typename cplx_
         };
 #pragma unroll
         for (int k = 0; k < H; ++k) {
-            const RegRot<T> q = r[k];
+            const RegRot q = r[k];
             columns(a[k], a[NP - 1 - k], q);
             columns(v[k], v[NP - 1 - k], q);
         }
         // Row rotation: lower row <- c own - s partner, upper row <- c own + conj(s) partner.
-        const T wx = upper ? s.x : -s.x, wy = -s.y;
+        const double wx = upper ? s.x : -s.x, wy = -s.y;
 #pragma unroll
         for (int j = 0; j < NP; ++j) {
-            const T px = G::from(a[j].x, partner), py = G::from(a[j].y, partner);
+            const double px = G::from(a[j].x, partner), py = G::from(a[j].y, partner);
             a[j].x = fma(-wy, py, fma(wx, px, c * a[j].x));
             a[j].y = fma(wy, px, fma(wx, py, c * a[j].y));
         }
         if constexpr (NP > 2) {
-            const C a1 = a[1], v1 = v[1];
+            const double2 a1 = a[1], v1 = v[1];
 #pragma unroll
             for (int j = 1; j < NP - 1; ++j) { a[j] = a[j + 1]; v[j] = v[j + 1]; }
             a[NP - 1] = a1;
@@ -151,24 +144,24 @@ WNLQG_D bool reg_jacobi_sweep(typename cplx_of<T>::type (&a)[NP], typename cplx_
 }
 
 // Squared off-diagonal norm of the group's matrix (slot s holding index s).
-template <typename T, int NP> WNLQG_D T reg_offdiag2(const typename cplx_of<T>::type (&a)[NP]) {
+template <int NP> WNLQG_D double reg_offdiag2(const double2 (&a)[NP]) {
     const int i = RegGroup<NP>::lane();
-    T s = (T)0;
+    double s = 0.0;
 #pragma unroll
-    for (int j = 0; j < NP; ++j) s += j == i ? (T)0 : a[j].x * a[j].x + a[j].y * a[j].y;
-    return RegGroup<NP>::sum(i < NP ? s : (T)0);
+    for (int j = 0; j < NP; ++j) s += j == i ? 0.0 : a[j].x * a[j].x + a[j].y * a[j].y;
+    return RegGroup<NP>::sum(i < NP ? s : 0.0);
 }
 
-// Shared memory of one group: S matrices of NP rows of LD complex entries (16-byte rows), rotations.
-template <typename T, int NP, int S> struct RegSmem {
-    typedef typename cplx_of<T>::type C;
+// Shared memory of one group: a matrix of NP rows of LD complex entries (16-byte rows), rotations.
+template <int NP> struct RegSmem {
     static constexpr int LD = NP + 2;
-    C m[S][NP * LD];
-    RegRot<T> rot[NP];
+    double2 m[NP * LD];
+    RegRot rot[NP];
 };
 
 // Upper triangle of a stored Hermitian matrix into shared rows S[i * LD + j] (lower = conjugate, real
-// diagonal, zeros beyond nw); valid = 0 stores zeros.  Closes with __syncwarp.
+// diagonal, zeros beyond nw), here in FP64 and in FP32 for the one-sided stage (onesided.cuh); valid = 0
+// stores zeros.  Closes with __syncwarp.
 template <typename T, int NP>
 WNLQG_D void reg_stage_hermitian(typename cplx_of<T>::type *S, const double2 *__restrict__ h, int nw, bool valid) {
     typedef typename cplx_of<T>::type C;
@@ -200,11 +193,11 @@ __global__ void __launch_bounds__(128, NP > 8 ? 2 : 3) jacobi_f64_reg_kernel(
     const double2 *__restrict__ h_in, int64_t h_stride, int64_t batch, int nw, double *__restrict__ E_out,
     double2 *__restrict__ U_out) {
     typedef RegGroup<NP> G;
-    typedef RegSmem<double, NP, 1> Smem;
+    typedef RegSmem<NP> Smem;
     constexpr int LD = Smem::LD;
     extern __shared__ __align__(16) unsigned char reg_smem_raw[];
     Smem &sm = reinterpret_cast<Smem *>(reg_smem_raw)[threadIdx.x / G::LANES];
-    double2 *S = sm.m[0];
+    double2 *S = sm.m;
     const int i = G::lane(), ic = min(i, NP - 1);
     const int64_t groups = (int64_t)gridDim.x * blockDim.x / G::LANES;
     const int64_t g = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / G::LANES;
@@ -226,11 +219,11 @@ __global__ void __launch_bounds__(128, NP > 8 ? 2 : 3) jacobi_f64_reg_kernel(
         const double stop = tol * NP;
         bool done = !valid;
         for (int sweep = 0; sweep < 30; ++sweep) {
-            const double off = sqrt(reg_offdiag2<double, NP>(a));   // every lane takes the shuffles
+            const double off = sqrt(reg_offdiag2<NP>(a));   // every lane takes the shuffles
             done = done || off <= stop;
             if (__all_sync(0xffffffffu, done)) break;
             if (done) tol = 1.0e150;   // nothing rotates
-            const bool any = reg_jacobi_sweep<double, NP>(a, v, d, tol, sm.rot);
+            const bool any = reg_jacobi_sweep<NP>(a, v, d, tol, sm.rot);
             done = done || !any;
         }
         // Lane i: rank of eigenvalue i (ascending, ties in index order), pivot and phase of its column.
@@ -274,7 +267,7 @@ struct RegKernel {
     int lanes;
 };
 template <int NP> RegKernel reg_f64_entry() {
-    return {(const void *)jacobi_f64_reg_kernel<NP>, sizeof(RegSmem<double, NP, 1>), RegGroup<NP>::LANES};
+    return {(const void *)jacobi_f64_reg_kernel<NP>, sizeof(RegSmem<NP>), RegGroup<NP>::LANES};
 }
 inline RegKernel reg_f64_kernel(int np) {
     static const RegKernel k[8] = {reg_f64_entry<2>(),  reg_f64_entry<4>(),  reg_f64_entry<6>(),  reg_f64_entry<8>(),

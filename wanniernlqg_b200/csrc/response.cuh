@@ -144,7 +144,7 @@ struct RespSmem {
         s.E = take(nw * sizeof(double));
         s.f = take(nw * sizeof(double));
         s.te = take((size_t)nw * nw * sizeof(double));
-        s.fnm = take((size_t)nw * nw * sizeof(double));
+        s.fnm = take(((size_t)nw * nw + (nw == 1)) * sizeof(double));   // room for nw + 1 Hall sums
         s.Q = take((size_t)nw * nw * n_fc * csize);
         s.fd = take((size_t)4 * nw * (n_berry > 0 ? n_berry : 1) * sizeof(double2));
         s.hess = take((size_t)RS_MAX_HESS * nw * sizeof(double));
@@ -614,7 +614,8 @@ __global__ void __launch_bounds__(WIDE ? 512 : 256, WIDE ? 1 : (sizeof(R) == 8 &
             //   sum_AD + AD_bit = [A_p, D_d]_nm + (A_d,nn - A_d,mm) D_p,nm
             //   sum_HD + DV_bit = [dH_p, D_d]_nm + (dH_d,nn - dH_d,mm) D_p,nm
             // The pair-data region (transition energies, occupations, pair kernels: at least
-            // 32 nw^2 bytes) is unused until the pairs are built, so it holds the rotated ddH.
+            // 32 nw^2 bytes, as a pass with generalised derivatives has a frequency component) is
+            // unused until the pairs are built, so it holds the rotated ddH.
             C *Hpd = reinterpret_cast<C *>(sm + L.te);
             for (int g = 0; g < p.n_g; ++g) {
                 const int pp = p.g_p[g], dd = p.g_d[g];
@@ -697,8 +698,9 @@ __global__ void __launch_bounds__(WIDE ? 512 : 256, WIDE ? 1 : (sizeof(R) == 8 &
         // component in the pair-data region (free until the pairs are built); the Fermi levels then
         // only combine it: a warp per level (dipole, linear transport) or a thread per level (AHC).
         // Bound before by barriers and serial sums (a block sum per level, the dipole's levels on one
-        // thread): a 201-level Hall scan of 18 orbitals, 2025 points, took 2.43 ms and takes 0.70;
-        // transport and dipole at 3 levels, 24 orbitals, 32768 points, 21.2 ms and 11.6.
+        // thread): a 201-level Hall scan of 18 orbitals, 2025 points, 2.43 -> 0.70 ms; transport and dipole
+        // at 3 levels, 24 orbitals, 32768 points, 21.2 -> 11.6 (whole calls, with the eigensolver they had then;
+        // 0.58 and 9.0 with the present one).
         const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
         auto mu_emit = [&](int64_t idx, double value) {
             if (p.mode == 0) {

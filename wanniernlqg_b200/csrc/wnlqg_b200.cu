@@ -1046,7 +1046,7 @@ wnlqg_status run_front(wnlqg_plan *pl, int64_t nb, int64_t k_begin, const int64_
     if (st != WNLQG_OK) return st;
     const unsigned eigh_grid = (unsigned)(pl->d_eigh_scratch ? std::min<int64_t>(nb, pl->eigh_grid) : nb);
     if (pl->nonorth && pl->gen_mixed) {
-        // FP64 Cholesky reduction, the orthogonal mixed-precision stages on C, U = L^-H V.
+        // FP64 Cholesky reduction, the orthogonal stages of the plan's precision on C, U = L^-H V.
         const double2 *hk = pl->d_xw + (int64_t)pl->ch_H * pl->nn, *sk = pl->d_xw + (int64_t)pl->ch_S * pl->nn;
         if (pl->gred_gw) {
             cholesky_reduce_kernel<true><<<(unsigned)std::min<int64_t>(nb, pl->gred_grid), 256, 0, pl->stream>>>(
@@ -2085,7 +2085,6 @@ wnlqg_status wnlqg_b200_plan_create(wnlqg_model *model, const wnlqg_task_desc *t
             if (ea == cudaSuccess) ea = allow_dynamic_smem((const void *)jacobi_f32_team_kernel<32>, smem_optin);
             if (ea == cudaSuccess) ea = allow_dynamic_smem((const void *)jacobi_f32_team_kernel<64>, smem_optin);
             if (ea == cudaSuccess) ea = allow_dynamic_smem((const void *)jacobi_f32_team_kernel<128>, smem_optin);
-            if (ea == cudaSuccess && pl->small_f64) ea = allow_dynamic_smem(reg_f64_kernel(np).fn, smem_optin);
             if (ea != cudaSuccess) return bail(fail(WNLQG_ERR_CUDA, std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(ea)));
         }
         // Both stages need blockDim >= np/2 (pairs) and 8 * blockDim >= np^2 (register-staged products).
